@@ -209,13 +209,28 @@ def _weights(case, n, k, dt, gen):
     return _words((bits, n, k // 32) if fmt == "anyprec" else (k * bits // 32, n), gen), lut
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """(n, k, channels compensated per 1024), activations, (residual, scales, thresholds) or None, weights: of every linear of a pass."""
     dt = DTYPES[case["dtype"]]
     gen = torch.Generator(device="cuda").manual_seed(seed)
+    linears, blocks = _linears(case)
+    xs = {k: _activation(k, dt, gen) for k in sorted({k for _, _, k, _ in linears})} if case["op"] == "decode" else {}
+    for _ in range(blocks):
+        for _, n, k, kc in linears:
+            compensation = None
+            if case["op"] == "decode" and case["comp"]:
+                residual = _words((k, n // 8), gen).cpu()
+                scales = (torch.rand(n, device="cuda", generator=gen) * 1e-3 + 2e-4).to(dt).cpu()
+                compensation = residual, scales, _thresholds(k, dt, gen)
+            yield (n, k, kc), xs.get(k), compensation, _weights(case, n, k, dt, gen)
+
+
+def prepare(case, seed):
+    dt = DTYPES[case["dtype"]]
     s = _State(case)
     linears, blocks = _linears(case)
     if case["op"] == "prefill":
-        s.layers = [_weights(case, n, k, dt, gen) for _ in range(blocks) for _, n, k, _ in linears]
+        s.layers = [weights for _, _, _, weights in _inputs(case, seed)]
         return s
     comp = case["comp"]
     if comp:
@@ -226,18 +241,14 @@ def prepare(case, seed):
     # one buffer for all outputs, so that one memset clears them; offsets keep each output 256-byte aligned
     pad = [(n + 127) // 128 * 128 for _, n, _, _ in linears]
     s.y = torch.zeros(blocks * sum(pad), dtype=dt, device="cuda")
-    x = {k: _activation(k, dt, gen) for k in sorted({k for _, _, k, _ in linears})}
     at = 0
-    for _ in range(blocks):
-        for (_, n, k, kc), room in zip(linears, pad):
-            cfg = None
-            if comp:
-                residual = _words((k, n // 8), gen).cpu()
-                scales = (torch.rand(n, device="cuda", generator=gen) * 1e-3 + 2e-4).to(dt).cpu()
-                cfg = ext.create_dec_config(ctx, kc, residual, scales, _thresholds(k, dt, gen))
-                s.configs.append(cfg)
-            s.layers.append((cfg, x[k], s.y[at:at + n].view(1, 1, n), _weights(case, n, k, dt, gen)))
-            at += room
+    for (n, k, kc), x, compensation, weights in _inputs(case, seed):
+        cfg = None
+        if comp:
+            cfg = ext.create_dec_config(ctx, kc, *compensation)
+            s.configs.append(cfg)
+        s.layers.append((cfg, x, s.y[at:at + n].view(1, 1, n), weights))
+        at += (n + 127) // 128 * 128
     if case["graph"]:
         stream = torch.cuda.Stream() if prepare.stream is None else prepare.stream
         prepare.stream = stream
@@ -287,4 +298,84 @@ def run(s):
     out = [layer[2] for layer in s.layers]
     if s.case["comp"] and s.selected:
         out += [s.rows[: s.selected], s.acts[: s.selected]]
+    return out
+
+
+# ---- the same results in 64 bits, without the library ----------------------------------------------------------------
+
+def _dense(case, n, k, w):
+    """[n, k] weights in 64 bits, from the packed tensors as their formats are documented."""
+    bits, dev = case["bits"], "cuda"
+    if case["fmt"] == "bcq":                       # words [k / 32, bits, n], bit i = channel i of the word: sum of +-alpha, plus the bias
+        words, alpha, bias = w
+        shifts = torch.arange(32, device=dev).view(1, 32, 1)
+        dense = bias.double().repeat_interleave(case["group"], 0)
+        for p in range(bits):
+            signs = (((words[:, p].unsqueeze(1) >> shifts) & 1) * 2 - 1).view(k, n)
+            dense += signs * alpha[:, p].double().repeat_interleave(case["group"], 0)
+        return dense.t()
+    words, lut = w
+    if case["fmt"] == "anyprec":                   # planes [bits, n, k / 32], most significant first, channels interleaved within 1024
+        channel = torch.empty(k, dtype=torch.long)
+        for at in range(0, k, 1024):
+            e = min(1024, k - at) // 32
+            t, j, r = torch.meshgrid(torch.arange(e), torch.arange(4), torch.arange(8), indexing="ij")
+            channel[at:at + 32 * e] = (at + 8 * e * j + 8 * t + r).reshape(-1)
+        shifts = torch.arange(31, -1, -1, device=dev)
+        codes = torch.zeros((n, k), dtype=torch.long, device=dev)
+        for p in range(bits):
+            codes = codes * 2 + ((words[p].unsqueeze(-1) >> shifts) & 1).view(n, k)
+        dense = torch.empty((n, k), dtype=torch.float64, device=dev)
+        dense[:, channel.to(dev)] = lut.double().gather(1, codes)
+        return dense
+    # 32 channels are one little-endian string of codes in `bits` words of a column
+    string = ((words.view(k // 32, bits, 1, n) >> torch.arange(32, device=dev).view(1, 1, 32, 1)) & 1).view(k, bits, n)
+    codes = (string.long() << torch.arange(bits, device=dev).view(1, bits, 1)).sum(1)
+    return lut.double().gather(1, codes.t())
+
+
+def _selection(x, thresholds, kc):
+    """Channels that are compensated: per 1024 the kc of the highest buckets, the lowest indices of the last bucket."""
+    k, dt = x.numel(), x.dtype
+    a, b = thresholds[0], thresholds[max(0, kc * k // 1024 - 1)]
+    level = torch.arange(32)
+    upper = a + ((b - a).float() * level / 15).to(dt)
+    lower = (b.float() * (31 - level) / 16).to(dt)
+    floors = torch.where(level < 16, upper, lower).float()
+    rows = []
+    for at in range(0, k, 1024):
+        mag = x[at:at + 1024].float().abs().cpu()
+        over = mag.unsqueeze(1) >= floors
+        bucket = torch.where(over.any(1), over.int().argmax(1), 32)
+        rows.append(at + bucket.sort(stable=True).indices[: kc * mag.numel() // 1024])
+    return torch.cat(rows).cuda()
+
+
+def exact(case, seed):
+    """The outputs of `run`; nothing for the selection that is returned beside them (whole numbers and copies), nor for the
+    dense weights of a prefill, which are compared bit by bit."""
+    if case["op"] == "prefill":
+        return None
+    out = []
+    for (n, k, kc), x, comp, w in _inputs(case, seed):
+        xd = x.reshape(-1).double()
+        step = max(8, (1 << 27) // k // 8 * 8)
+        parts = []
+        for n0 in range(0, n, step):
+            n1 = min(n, n0 + step)
+            if case["fmt"] == "bcq":
+                piece = (w[0][:, :, n0:n1], w[1][:, :, n0:n1], w[2][:, n0:n1])
+            else:
+                piece = (w[0][:, n0:n1], w[1][n0:n1])
+            parts.append(_dense(case, n1 - n0, k, piece) @ xd)
+        y = torch.cat(parts)
+        if comp is not None and kc * k // 1024:
+            residual, scales, thresholds = comp
+            rows = _selection(x.reshape(-1), thresholds, kc)
+            nibbles = (residual.cuda()[rows].unsqueeze(-1) >> (4 * torch.arange(8, device="cuda"))) & 15
+            by_output = scales.cuda().double().view(8, n // 8).t().reshape(-1)      # stored [output % 8][output / 8]
+            y += (xd[rows] @ (nibbles.double() - 8).view(-1, n)) * by_output
+        out.append(y.view(1, 1, n))
+    if case["comp"] and _linears(case)[0][-1][3] * _linears(case)[0][-1][2] // 1024:
+        out += [None, None]
     return out
