@@ -18,6 +18,7 @@
 #pragma once
 #include "gemv_anyprec.cuh"
 #include "gemv_bcq_pipe.cuh"
+#include "lut_bytes.cuh"
 
 namespace dd {
 
@@ -38,23 +39,6 @@ struct ApPipeGeom {
 };
 
 constexpr int kApPipeHdr = 256;   // [abort, flag][full barriers 8][empty barriers 8]
-
-// 4-bit fields from up to four plane words: field t (bits 4t..4t+3) of result ph holds, most significant plane
-// first, the bits that planes P[0..B-1] carry at position 4t + ph.
-template <int B>
-__device__ __forceinline__ void ap_fields(const uint32_t* P, uint32_t (&V)[4]) {
-    uint32_t R[B];
-#pragma unroll
-    for (int i = 0; i < B; ++i) R[i] = i ? __funnelshift_r(P[i], P[i], i) : P[0];
-#pragma unroll
-    for (int ph = 0; ph < 4; ++ph) {
-        uint32_t m = 0u;
-#pragma unroll
-        for (int i = 0; i < B; ++i) m |= R[i] & (0x11111111u << ((ph - i) & 3));
-        const int rot = (B - 1 - ph) & 31;
-        V[ph] = rot ? __funnelshift_l(m, m, rot) : m;
-    }
-}
 
 // d += a * b with 16-bit factors (raw bits of the element type) and an fp32 accumulator
 template <int DT>

@@ -144,13 +144,36 @@ cudaError_t launch_anyprec_pipe(int dt, const ApParams& g, const DecParams& d, c
     return dt == FP16 ? pipe_by_bits<FP16>(g, d, f, geo, s) : pipe_by_bits<BF16>(g, d, f, geo, s);
 }
 
+template <int DT, int BITS>
+static void dequant_bits(int blocks, const uint32_t* qweight, const void* lut, void* out, uint32_t N, uint32_t K, cudaStream_t s) {
+    if constexpr (BITS <= 4) {
+        if ((reinterpret_cast<uintptr_t>(lut) & 15u) == 0u) {        // the table rows are read with 16-byte loads
+            ap_dequant_kernel<DT, BITS, true><<<blocks, kThreads, 0, s>>>(qweight, lut, out, N, K);
+            return;
+        }
+    }
+    ap_dequant_kernel<DT, BITS, false><<<blocks, kThreads, 0, s>>>(qweight, lut, out, N, K);
+}
+
+template <int DT>
+static void dequant_dt(int blocks, const uint32_t* qweight, const void* lut, void* out, uint32_t N, uint32_t K, uint32_t bits, cudaStream_t s) {
+    switch (bits) {
+        case 3: dequant_bits<DT, 3>(blocks, qweight, lut, out, N, K, s); break;
+        case 4: dequant_bits<DT, 4>(blocks, qweight, lut, out, N, K, s); break;
+        case 5: dequant_bits<DT, 5>(blocks, qweight, lut, out, N, K, s); break;
+        case 6: dequant_bits<DT, 6>(blocks, qweight, lut, out, N, K, s); break;
+        case 7: dequant_bits<DT, 7>(blocks, qweight, lut, out, N, K, s); break;
+        default: dequant_bits<DT, 8>(blocks, qweight, lut, out, N, K, s); break;
+    }
+}
+
 cudaError_t launch_ap_dequant(int dt, const uint32_t* qweight, const void* lut, void* out, uint32_t N, uint32_t K,
                               uint32_t bits, cudaStream_t s) {
     const size_t total = (size_t)N * (K / 32);
     const int blocks = (int)((total + kThreads - 1) / kThreads < 148 * 16 ? (total + kThreads - 1) / kThreads : 148 * 16);
     if (blocks == 0) return cudaSuccess;
-    if (dt == FP16) ap_dequant_kernel<FP16><<<blocks, kThreads, 0, s>>>(qweight, lut, out, N, K, bits);
-    else ap_dequant_kernel<BF16><<<blocks, kThreads, 0, s>>>(qweight, lut, out, N, K, bits);
+    if (dt == FP16) dequant_dt<FP16>(blocks, qweight, lut, out, N, K, bits, s);
+    else dequant_dt<BF16>(blocks, qweight, lut, out, N, K, bits, s);
     return cudaGetLastError();
 }
 

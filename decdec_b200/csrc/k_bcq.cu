@@ -187,12 +187,31 @@ cudaError_t launch_bcq(int dt, const BcqParams& g, const DecParams& d, const Fin
     }
 }
 
+template <int DT>
+static void dequant_vec(int blocks, const uint32_t* qweight, const void* alpha, const void* q_bias, void* out, uint32_t N,
+                        uint32_t K, uint32_t bits, uint32_t group, cudaStream_t s) {
+    switch (bits) {
+        case 1: bcq_dequant_vec_kernel<DT, 1><<<blocks, kThreads, 0, s>>>(qweight, alpha, q_bias, out, N, K, group); break;
+        case 2: bcq_dequant_vec_kernel<DT, 2><<<blocks, kThreads, 0, s>>>(qweight, alpha, q_bias, out, N, K, group); break;
+        case 3: bcq_dequant_vec_kernel<DT, 3><<<blocks, kThreads, 0, s>>>(qweight, alpha, q_bias, out, N, K, group); break;
+        default: bcq_dequant_vec_kernel<DT, 4><<<blocks, kThreads, 0, s>>>(qweight, alpha, q_bias, out, N, K, group); break;
+    }
+}
+
 cudaError_t launch_bcq_dequant(int dt, const uint32_t* qweight, const void* alpha, const void* q_bias, void* out, uint32_t N,
                                uint32_t K, uint32_t bits, uint32_t group, cudaStream_t s) {
-    const size_t total = (size_t)(K / 32) * (N / 2);
+    // four outputs per thread where 16-byte loads of the planes, 8-byte loads of the scales and 8-byte stores are aligned
+    const bool vec = dt != FP32 && bits <= 4 && N % 4u == 0u && (reinterpret_cast<uintptr_t>(qweight) & 15u) == 0u &&
+                     ((reinterpret_cast<uintptr_t>(alpha) | reinterpret_cast<uintptr_t>(q_bias) | reinterpret_cast<uintptr_t>(out)) & 7u) == 0u;
+    const size_t total = (size_t)(K / 32) * (N / (vec ? 4 : 2));
     const size_t want = (total + kThreads - 1) / kThreads;
     const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
     if (blocks == 0) return cudaSuccess;
+    if (vec) {
+        if (dt == FP16) dequant_vec<FP16>(blocks, qweight, alpha, q_bias, out, N, K, bits, group, s);
+        else dequant_vec<BF16>(blocks, qweight, alpha, q_bias, out, N, K, bits, group, s);
+        return cudaGetLastError();
+    }
     switch (dt) {
         case FP32: bcq_dequant_kernel<FP32><<<blocks, kThreads, 0, s>>>(qweight, alpha, q_bias, out, N, K, bits, group); break;
         case FP16: bcq_dequant_kernel<FP16><<<blocks, kThreads, 0, s>>>(qweight, alpha, q_bias, out, N, K, bits, group); break;
