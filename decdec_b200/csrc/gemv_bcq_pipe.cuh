@@ -28,8 +28,11 @@
 // cluster placement delays the early start that programmatic dependent launch gives, and walking several K slices
 // per CTA costs about 1.5 us per table rebuild.
 //
-// Requirements (otherwise the register-staged kernel of gemv_bcq.cuh runs): N % 128 == 0,
-// K % 512 == 0, group size one of 32..512 dividing 512, at least two stages fit in shared memory.
+// Ragged shapes: a box that reaches beyond the tensor's last output or word row is filled with zeros by the copy (and counts
+// its full bytes), so the planes, alpha and q_bias of outputs and channels that do not exist are zero; activations beyond K
+// are zero in the tables, and only outputs below N are added.
+// Requirements (otherwise the register-staged kernel of gemv_bcq.cuh runs): 2 to 4 bits, group size one of 32..512 dividing
+// 512, N % 8 == 0 (row strides of the tensor maps), at least two stages fit in shared memory.
 // Every wait (mbarrier, tile counter) is bounded; on expiry the CTA raises the error word of the workspace, still
 // takes part in the counter / ticket protocol (so that the workspace stays consistent) and the caller reads the
 // error through decdec_stream_status.
@@ -189,7 +192,7 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
     const uint32_t ks = cta % p.n_kslices;
     const uint32_t tile = cta / p.n_kslices;
     const uint32_t kbase = ks * kBcqSlice;
-    const uint32_t nst_total = p.N / kPipeStageN;
+    const uint32_t nst_total = (p.N + kPipeStageN - 1) / kPipeStageN;
     const uint32_t st0 = tile * geo.tile_stages;
     const uint32_t nst = min(geo.tile_stages, nst_total - st0);
     const uint32_t S = geo.stages;
@@ -281,7 +284,6 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
         const bool swapAB = (tA & 4) != 0;                  // after the swap X = group r, Y = group r + 4, r = tA & 3
         const uint32_t r4 = tA & 3;
         const uint32_t n_out = blk * 32 + ((j & 4) ? 16 : 0) + 4 * r4 + (j & 3);
-        float* acc_lane = f.acc + (size_t)st0 * kPipeStageN + n_out;
         bool pending = false;
         unsigned long long p_old = 0, p_mine = 0;
         unsigned long long* p_word = nullptr;
@@ -290,8 +292,8 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
 
         pdl_wait();     // weights are already streaming (producer warp); activations come from earlier kernels
         if (builder && !*s_abort) {
-            float xv[8];
-            pipe_load_x8<DT>(p.x, kbase + koff, xvec, xv);
+            float xv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (kbase + koff < p.K) pipe_load_x8<DT>(p.x, kbase + koff, xvec, xv);     // K is a multiple of 32
             float lo[8], hi[4];
 #pragma unroll
             for (int e = 0; e < 8; ++e)
@@ -366,12 +368,12 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
                 const float keep = (j & 1) ? y2[1] : y2[0];
                 y1 = keep + __shfl_sync(0xffffffffu, send, p1);
             }
+            const uint32_t n = (st0 + i) * kPipeStageN + n_out;
             if (!geo.packed) {
-                atomicAdd(acc_lane + i * kPipeStageN, y1);
+                if (n < p.N) atomicAdd(f.acc + n, y1);
             } else {
                 // the previous stage's atomic has long returned: settle it, then send this stage's
                 if (pending) finish_packed<DT>(p_old, p_mine, geo.arrivals, p_word, p_y, p_y0);
-                const uint32_t n = (st0 + i) * kPipeStageN + n_out;
                 p_word = reinterpret_cast<unsigned long long*>(f.acc) + n;
                 p_y = reinterpret_cast<T*>(f.y) + n;
                 p_y0 = Tr<DT>::to_f(*p_y);

@@ -339,8 +339,9 @@ int run_bcq(Config* c, const void* x, void* y, const int32_t* qw, const void* al
     }
     // Launches of the pipelined kernel carry sums and arrival counts in one 64-bit atomic per output (the accumulator
     // allocation holds kAccCap such words) instead of tickets; DECDEC_BCQ_PACKED=0 keeps the ticket protocol.  With a
-    // compensation role the CTA's private cells must fit in shared memory beside the selection state.
-    if (pipe && env_u32("DECDEC_BCQ_PACKED", 1)) {
+    // compensation role the CTA's private cells must fit in shared memory beside the selection state.  Ragged layers keep the
+    // fp32 accumulator and tickets: the words' fixed point has an absolute resolution that their sums never had.
+    if (pipe && N % kPipeStageN == 0u && K % kBcqSlice == 0u && env_u32("DECDEC_BCQ_PACKED", 1)) {
         const uint32_t arrivals = 2u * g.n_kslices + (d.n_cta ? d.n_rowparts : 0u);
         bool ok = arrivals <= 255u;
         if (ok && d.n_cta) {

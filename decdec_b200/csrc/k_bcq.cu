@@ -136,7 +136,7 @@ static uint32_t env_u32_k(const char* name, uint32_t dflt) {
 // sm_budget = SMs the GEMV CTAs may fill in one wave.
 bool bcq_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, uint32_t group, int dt, uint32_t n_kslices, PipeGeom* geo,
                        uint32_t sm_budget) {
-    if (N % kPipeStageN || K % kBcqSlice || bits < 2 || bits > 4) return false;
+    if (N % 8u || K % 32u || bits < 2 || bits > 4) return false;      // ragged ends are filled with zeros by the copies
     if (group < 32 || group > (uint32_t)kBcqSlice || kBcqSlice % group) return false;
     // the table block sits at the first 64 KB multiple of the shared window; dynamic shared memory starts right
     // after the bytes the system reserves per CTA (this kernel has no static shared memory)
@@ -155,7 +155,7 @@ bool bcq_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, uint32_t group, in
     uint32_t smax = n_before + room_after / geo->stage_bytes;
     if (smax > 8) smax = 8;
     if (smax < 2) return false;
-    const uint32_t nst_total = N / kPipeStageN;
+    const uint32_t nst_total = (N + kPipeStageN - 1) / kPipeStageN;
     // one CTA per SM; tiles sized so that the grid is at most one wave
     uint32_t per1 = sm_budget / n_kslices; if (per1 == 0) per1 = 1;
     geo->tile_stages = (nst_total + per1 - 1) / per1;

@@ -1,6 +1,8 @@
-"""Edges of the table-lookup kernels on the GPU: the vector forms of the dequantizers against the arithmetic they stand for.
+"""Edges of the table-lookup kernels on the GPU: ragged layers, vector dequantizers.
 
-Oracle: the dense weights of the packed tensors; compared bit by bit.
+Oracle: the dense weights of the packed tensors in float64.  Tolerances of the GEMVs: products and sums are fp32, and the output is rounded once; with y = 0 before the call the error of an output is at most
+half an ulp of it (2^-11 or 2^-8 of its size in fp16 and bf16) plus the fp32 sum's, K * 2^-24 of the sum of magnitudes, which
+the bound below takes at its worst.  Dense weights are compared exactly.
 """
 import numpy as np
 import pytest
@@ -16,6 +18,38 @@ def ops():
     assert torch.cuda.is_available(), "GPU tests need a CUDA device"
     from decdec_b200 import ops as _ops
     return _ops
+
+
+HALF_ULP = {"fp16": 2.0 ** -11, "bf16": 2.0 ** -8, "fp32": 2.0 ** -24}
+
+
+def _assert_sums(y, w_hat, x, dtype):
+    xd = P.to_np(x).reshape(-1)
+    ref = w_hat @ xd
+    mags = np.abs(w_hat) @ np.abs(xd)
+    bound = HALF_ULP[dtype] * np.abs(ref) + w_hat.shape[1] * 2.0 ** -24 * mags + 2.0 ** -24
+    worst = (np.abs(P.to_np(y).reshape(-1) - ref) / bound).max()
+    assert worst <= 1.0, f"error up to {worst:.2f} of its bound"
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16", "fp32"])
+@pytest.mark.parametrize("N,K,bits,group", [
+    (8, 32, 2, 32),          # a box larger than the tensor in every direction
+    (120, 480, 3, 32),       # one short tile, one short slice
+    (136, 544, 4, 32),       # one output tile and one slice, each with a remainder
+    (2776, 1184, 4, 32),
+    (3000, 4224, 3, 128),    # many tiles, the last slice a quarter full
+])
+def test_lutgemm_ragged_layers(ops, dtype, N, K, bits, group):
+    L = P.random_bcq_layer(N, K, bits, group, seed=N + K, dtype=dtype)
+    x = P.make_activation(K, seed=11, dtype=dtype)
+    big = torch.zeros(N + 256, dtype=P.TORCH_DT[dtype], device="cuda")
+    y = big[:N].view(1, 1, N)
+    for _ in range(2):                                   # the second call finds the workspace as the first left it
+        y.zero_()
+        ops.lutgemm_gemv(x.cuda(), y, L["qweight"].cuda(), L["alpha"].cuda(), L["q_bias"].cuda(), bits, group)
+        _assert_sums(y, L["w_hat"], x, dtype)
+        assert not big[N:].any()                         # nothing beyond the last output
 
 
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
