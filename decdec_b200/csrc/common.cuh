@@ -85,6 +85,27 @@ __device__ __forceinline__ uint32_t ldg_stream(const uint32_t* p) {
     return v;
 }
 
+// D += A * B with 16-bit factors and fp32 sums (mma.m16n8k16): a lane (g, t) = (lane / 4, lane % 4) holds A rows g (a0, a2) and
+// g + 8 (a1, a3) at k = 2t, 2t+1 (a0, a1) and 2t+8, 2t+9 (a2, a3), B column g at the same k (b0, b1), and D rows g (d[0], d[1])
+// and g + 8 (d[2], d[3]) at columns 2t, 2t+1.
+template <int DT>
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    static_assert(DT != FP32, "16-bit factors");
+    if constexpr (DT == FP16)
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// the two 16-bit values of a register
+template <int DT>
+__device__ __forceinline__ float2 unpack2(uint32_t v) {
+    if constexpr (DT == FP16) return __half22float2(*reinterpret_cast<const __half2*>(&v));
+    else return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+
 // Programmatic dependent launch: a kernel launched with the programmatic-serialization attribute may
 // start while the previous kernel of the stream is still draining.  `pdl_trigger` lets the NEXT
 // kernel's CTAs be scheduled early; `pdl_wait` blocks until the PREVIOUS kernel has completed and its
@@ -210,17 +231,18 @@ __device__ __forceinline__ void finalize_span(const FinParams& f, uint32_t n0, u
 // Must be called by all threads of the CTA, after all its reductions into the accumulators were issued.
 // `nthreads` = number of threads of the CTA that take part (threads beyond it must have exited; the
 // first warp always takes part).  The tickets of up to 32 tiles are taken by one warp in parallel, so a
-// CTA that covers many tiles pays one atomic round trip, not one per tile.
+// CTA that covers many tiles pays one atomic round trip, not one per tile.  `arrivals` = what this CTA counts for on each
+// of the tiles: a role whose CTAs share a tile unevenly counts the work they did, so that the sum per tile is fixed.
 template <int DT>
 __device__ __forceinline__ void arrive_and_finalize(const FinParams& f, uint32_t t0, uint32_t t1, unsigned* s_flag,
-                                                    uint32_t nthreads = kThreads) {
+                                                    uint32_t nthreads = kThreads, uint32_t arrivals = 1u) {
     __threadfence();
     __syncthreads();
     for (uint32_t tb = t0; tb < t1; tb += 32u) {
         if (threadIdx.x < 32u) {
             const uint32_t t = tb + threadIdx.x;
             bool last = false;
-            if (t < t1) last = (atomicAdd(&f.tickets[t], 1u) + 1u == f.expected);
+            if (t < t1) last = (atomicAdd(&f.tickets[t], arrivals) + arrivals == f.expected);
             const unsigned m = __ballot_sync(0xffffffffu, last);
             if (threadIdx.x == 0) *s_flag = m;
         }

@@ -8,7 +8,8 @@
 // A CTA owns 32 output columns for the whole of K: lane = column (128-byte coalesced word rows),
 // warp = K slice.  The column LUTs sit in shared memory as fp32 [code][column], so lane l always hits
 // bank l.  Sums are fp32; the eight K slices are combined in shared memory, so no cross-CTA
-// reduction is needed.
+// reduction is needed.  General form: fp32 layers, odd numbers of outputs and unaligned tensors; 16-bit layers take the
+// pair tables of gemv_sqllm_pair.cuh.
 #pragma once
 #include "common.cuh"
 
@@ -19,7 +20,7 @@ struct SqParams {
     const void* lut;           // [N, 2^bits]
     const void* x;             // [K]
     uint32_t K, N, bits;
-    uint32_t n_cta;            // ceil(N / 32)
+    uint32_t n_cta;            // ceil(N / 32); pair tables: thread blocks the work is cut over
     uint32_t direct;
 };
 

@@ -428,9 +428,18 @@ int run_sqllm(Config* c, const void* x, void* y, const int32_t* qw, const void* 
     g.lut = lut;
     g.x = x;
     g.K = K; g.N = N; g.bits = (uint32_t)bits;
+    // 16-bit layers with an even number of outputs take the pair tables; a tile counts K / 32 arrivals there
+    const bool pair = env_u32("DECDEC_SQ_PAIR", 1) && sqllm_pair_eligible(qw, lut, N, K, g.bits, dtype);
     FinParams f;
-    if (int r = setup_fin(&f, ws, y, N, 1, 1)) return r;
+    if (int r = setup_fin(&f, ws, y, N, pair ? kSqTileN / 32u : 1u, pair ? K / 32u : 1u)) return r;
     g.n_cta = f.n_tiles;
+    if (pair) {
+        // two thread blocks per SM hide each other's table builds, but none is made for less than sixteen groups
+        const uint64_t units = (uint64_t)f.n_tiles * (K / 32u);
+        uint64_t n = 2u * gemv_sm_budget(c, true);
+        if (n > (units + 15u) / 16u) n = (units + 15u) / 16u;
+        g.n_cta = (uint32_t)n;
+    }
     DecParams d;
     memset(&d, 0, sizeof(d));
     if (c) {
@@ -438,7 +447,8 @@ int run_sqllm(Config* c, const void* x, void* y, const int32_t* qw, const void* 
         if (d.n_cta) { f.expected += d.n_rowparts; f.acc2 = ws.acc2; f.scales = d.scales; }
     }
     g.direct = d.n_cta ? 0u : 1u;
-    DD_CUDA(launch_sqllm(dtype, g, d, f, s));
+    if (pair) DD_CUDA(launch_sqllm_pair(dtype, g, d, f, s));
+    else DD_CUDA(launch_sqllm(dtype, g, d, f, s));
     return 0;
 }
 

@@ -1,4 +1,4 @@
-"""Edges of the table-lookup kernels on the GPU: ragged layers, vector dequantizers.
+"""Edges of the table-lookup kernels on the GPU: ragged layers (binary-coded), pair tables (SqueezeLLM), vector dequantizers.
 
 Oracle: the dense weights of the packed tensors in float64.  Tolerances of the GEMVs: products and sums are fp32, and the output is rounded once; with y = 0 before the call the error of an output is at most
 half an ulp of it (2^-11 or 2^-8 of its size in fp16 and bf16) plus the fp32 sum's, K * 2^-24 of the sum of magnitudes, which
@@ -50,6 +50,41 @@ def test_lutgemm_ragged_layers(ops, dtype, N, K, bits, group):
         ops.lutgemm_gemv(x.cuda(), y, L["qweight"].cuda(), L["alpha"].cuda(), L["q_bias"].cuda(), bits, group)
         _assert_sums(y, L["w_hat"], x, dtype)
         assert not big[N:].any()                         # nothing beyond the last output
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("N,K", [
+    (2, 32),            # one pair of columns, one group
+    (64, 416),          # one tile, groups that do not fill the warps evenly
+    (66, 1024),         # a tile of two columns
+    (63, 256),          # odd: general kernel
+    (190, 8192),        # tiles cut over several thread blocks
+    (9600, 768),        # more tiles than thread blocks: whole tiles and cut ones
+])
+def test_sqllm_pair_tables(ops, dtype, bits, N, K):
+    L = P.lut_layer(N, K, bits, seed=N + K + bits, dtype=dtype, fmt="sqllm", real=False)
+    x = P.make_activation(K, seed=7, dtype=dtype)
+    for _ in range(2):                                   # the second call finds the workspace as the first left it
+        y = torch.zeros(1, 1, N, dtype=P.TORCH_DT[dtype], device="cuda")
+        ops.sqllm_gemv(x.cuda(), y, L["qweight"].cuda(), L["lut"].cuda(), bits)
+        _assert_sums(y, L["w_hat"], x, dtype)
+
+
+@pytest.mark.parametrize("bits", [3, 4])
+def test_sqllm_values_that_are_not_finite_stay_in_their_column(ops, bits):
+    N, K = 256, 1024
+    L = P.lut_layer(N, K, bits, seed=9, fmt="sqllm", real=False)
+    lut = L["lut"].clone()
+    lut[5, 1], lut[70, 2], lut[133, 0] = float("inf"), float("nan"), float("-inf")
+    x = P.make_activation(K, seed=7).abs() + 1
+    y = torch.zeros(1, 1, N, dtype=torch.float16, device="cuda")
+    ops.sqllm_gemv(x.cuda(), y, L["qweight"].cuda(), lut.cuda(), bits)
+    got = P.to_np(y).reshape(-1)
+    assert got[5] == np.inf and np.isnan(got[70]) and got[133] == -np.inf
+    rest = np.ones(N, bool)
+    rest[[5, 70, 133]] = False
+    _assert_sums(torch.from_numpy(got[rest]), L["w_hat"][rest], x, "fp16")
 
 
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
