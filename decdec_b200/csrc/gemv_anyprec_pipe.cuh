@@ -3,16 +3,25 @@
 // In the tensor [plane][row][K/32] consecutive rows of one plane are contiguous, so a stage of R rows is one
 // contiguous run per plane plus the R LUT rows.  A producer thread moves them with 1-D bulk asynchronous
 // copies (cp.async.bulk, completion counted on an mbarrier) several stages ahead of the consumer warps;
-// a warp's work item is (row of the stage, 4096-channel segment of that row).
-// Two decoders.  The 3-bit byte-permute decoder has the arithmetic of gemv_anyprec.cuh:ap3_role (register-
-// resident byte tables, activations staged in pair order).  The lookup decoder serves every width: the plane
-// words of 32 channels are regrouped into 4-bit fields with a handful of logic operations, each code indexes
-// the row's LUT where the bulk copy landed it in shared memory (a row of up to 64 entries spans at most 32 banks
-// and equal entries broadcast, so a warp's lookup is one wavefront), and the product goes into one of four fp32
-// sums with a mixed-precision multiply-add (16-bit factors, fp32 accumulator): no 16-bit partial sums.
-// A CTA owns its rows completely (all of K), so the row sums meet in a small shared-memory buffer and the
-// CTA folds them into y itself: GEMV-only launches use no global accumulator, ticket or fence.  Fused
-// launches store the sums into the workspace accumulator and arrive on the tile's ticket, where they meet
+// a warp's work item is (pair of rows of the stage, segment of their channels).
+// Bound: the ALU pipe (half of the issue rate): about 1.7 logic and permute operations turn a 3-bit code into its 16-bit weight,
+// 2.6 a 4-bit one.  Everything else is kept off that pipe:
+//  * the products go through mma.m16n8k16 (16-bit factors, fp32 sums; common.cuh): every lane supplies four weights of either
+//    row and its own four activations, lane (g, t) as rows g and g + 8 of A and column g of B, so that the diagonal entries
+//    D[g][g] and D[g + 8][g] hold the sums of the quad's lanes for the two rows; the other entries mix lanes and are not used.
+//    One instruction consumes eight weights per lane, and nothing is summed in 16 bits;
+//  * the eight diagonal sums of a row are stored, not shuffled together: the fold at the end adds a row's slots, in a fixed order;
+//  * the loop over a row's 1024-channel blocks is not unrolled (unrolled twice: the same times), and the last, shorter block has
+//    a body of its own, so that the masks it needs are not paid for by the others.
+// Measured, fp16, us per launch in a graph on 28672 x 4096, against the same stages with packed 16-bit sums (3 bits) or two
+// address operations and one mixed-precision multiply-add per weight (4 to 8 bits): 3 bits 24.2 -> 23.6, 4 bits 39.9 -> 30.0,
+// 5 bits 54.1 -> 33.8, 6 bits 55.5 -> 34.7, 8 bits 61.2 -> 57.9 (1.9, 2.0, 2.2, 2.6 and 2.3 TB/s of algorithmic bytes).
+// Two decoders.  3 bits: the row's table lives in registers and is looked up by byte permutes (lut_bytes.cuh), activations staged
+// in the pair order the lookups produce.  4 to 8 bits: the plane words are regrouped into 4-bit fields, each code indexes the
+// row's LUT in shared memory (a row of up to 64 entries spans at most 32 banks and equal entries broadcast, so a
+// lookup is one wavefront).
+// A CTA owns its rows completely (all of K) and folds them into y itself: GEMV-only launches use no global accumulator, ticket
+// or fence.  Fused launches store the sums into the workspace accumulator and arrive on the tile's ticket, where they meet
 // the compensation CTAs.
 // Requirements: K % 128 == 0, K <= 32768.  Every mbarrier wait is bounded.
 #pragma once
@@ -26,13 +35,14 @@ constexpr int kApPipeThreads = 544;   // 16 consumer warps + 1 producer warp
 
 struct ApPipeGeom {
     uint32_t rows_per_stage;   // R
-    uint32_t segs;             // ceil(K / 4096): warps per row
+    uint32_t segs;             // warps per pair of rows
+    uint32_t seg_words;        // plane words (32 channels each) of a row that one warp takes: a multiple of 32
     uint32_t stages;           // pipeline depth
     uint32_t stage_bytes;
-    uint32_t lookup;           // 1: lookup decoder, 0: byte-permute decoder (3 bits only)
     uint32_t x_bytes;          // staged activations (rounded to 128)
     uint32_t rows_per_cta;     // multiple of R
-    uint32_t part_bytes;       // row sums of the CTA (fp32, rounded to 128 bytes)
+    uint32_t part_bytes;       // partial sums of the CTA: fp32 [row][segment][8]
+    uint32_t lut_off;          // where the lookup decoder's warps keep their LUT rows (aligned to kApLutStride)
     uint32_t smem_bytes;
     uint32_t direct;           // 1: fold into y; 0: store into the accumulator and take the tile's ticket
     uint32_t wait_ns;          // limit of one mbarrier wait (DECDEC_PIPE_WAIT_NS)
@@ -40,48 +50,52 @@ struct ApPipeGeom {
 
 constexpr int kApPipeHdr = 256;   // [abort, flag][full barriers 8][empty barriers 8]
 
-// d += a * b with 16-bit factors (raw bits of the element type) and an fp32 accumulator
-template <int DT>
-__device__ __forceinline__ void ap_mixed_fma(float& d, uint16_t a, uint16_t b) {
-    if constexpr (DT == FP16) asm("fma.rn.f32.f16 %0, %1, %2, %0;" : "+f"(d) : "h"(a), "h"(b));
-    else asm("fma.rn.f32.bf16 %0, %1, %2, %0;" : "+f"(d) : "h"(a), "h"(b));
-}
+// One plane-word position (32 channels) of one row through the lookup decoder: W[jj][i] = weights of channels 2i (low half) and
+// 2i + 1 of group jj, beside the activations as they lie in memory.  `lut` is the window address of the row's LUT, aligned to
+// kApLutStride.  Up to 7 bits the byte offset of an entry, 2 * code, fits a byte: even and odd nibble positions are moved
+// into the bytes of two words (E and O), and one byte permute puts such a byte under the upper bytes of `lut`.
+template <int BITS> constexpr uint32_t kApLutStride = BITS <= 7 ? 256u : 512u;
 
-// One plane-word position (32 channels) of one row through the lookup decoder.  `lutrow` is the row's LUT where the
-// bulk copy landed it; X[j] holds the activations of channels 8 * E * j + (0..7) of the word's group.
-template <int DT, int BITS>
-__device__ __forceinline__ void ap_lookup_word(const uint32_t* q, const unsigned char* lutrow, const uint4 (&X)[4], float (&acc)[4]) {
+template <int BITS>
+__device__ __forceinline__ void ap_lookup_word(const uint32_t* q, uint32_t lut, uint32_t (&W)[4][4]) {
     constexpr int BH = BITS < 4 ? BITS : 4, BL = BITS - BH;
-    uint32_t Vh[4], Vl[4] = {0u, 0u, 0u, 0u};
-    ap_fields<BH>(q, Vh);
-    if constexpr (BL > 0) ap_fields<BL>(q + 4, Vl);
+    uint32_t Mh[4], Ml[4] = {0u, 0u, 0u, 0u}, E[4], O[4];
+    ap_merge<BH>(q, Mh);
+    if constexpr (BL > 0) ap_merge<BL>(q + 4, Ml);
+    constexpr uint32_t mh = 0x01010101u * (((1u << BH) - 1u) << (BITS <= 7 ? BL + 1 : BL)), ml = 0x01010101u * (((1u << BL) - 1u) << (BITS <= 7 ? 1 : 0));
 #pragma unroll
     for (int ph = 0; ph < 4; ++ph) {
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int pos = 31 - (4 * t + ph);          // channel = 8 * E * (pos / 8) + pos % 8 inside the word's group
-            const int jj = pos >> 3, r = pos & 7;
-            uint32_t off;                                // byte offset of the code's entry: 2 * code
-            if constexpr (BL == 0) {
-                off = t ? ((Vh[ph] >> (4 * t - 1)) & 0x1eu) : ((Vh[ph] << 1) & 0x1eu);
-            } else {
-                constexpr uint32_t mh = 0xfu << (BL + 1), ml = ((1u << BL) - 1u) << 1;
-                const int sh = 4 * t - BL - 1;
-                off = (sh >= 0) ? ((Vh[ph] >> (sh & 31)) & mh) : ((Vh[ph] << ((-sh) & 31)) & mh);
-                off |= t ? ((Vl[ph] >> (4 * t - 1)) & ml) : ((Vl[ph] << 1) & ml);
-            }
-            const uint16_t w = *reinterpret_cast<const uint16_t*>(lutrow + off);
-            const uint32_t xw = (&X[jj].x)[r >> 1];
-            const uint16_t xv = (r & 1) ? (uint16_t)(xw >> 16) : (uint16_t)(xw & 0xffffu);
-            ap_mixed_fma<DT>(acc[t & 3], w, xv);
+        const int rh = BH - 1 - ph + (BITS <= 7 ? BL + 1 : BL), rl = BL - 1 - ph + (BITS <= 7 ? 1 : 0);
+        E[ph] = rotate_left(Mh[ph], rh) & mh;
+        O[ph] = rotate_left(Mh[ph], rh - 4) & mh;
+        if constexpr (BL > 0) {
+            E[ph] |= rotate_left(Ml[ph], rl) & ml;
+            O[ph] |= rotate_left(Ml[ph], rl - 4) & ml;
         }
     }
+    auto entry = [&](int ph, int t) -> uint32_t {          // entry of the code at bit 4t + ph
+        const uint32_t src = (t & 1) ? O[ph] : E[ph];
+        const int b = t >> 1;
+        uint32_t addr;
+        if constexpr (BITS <= 7) addr = __byte_perm(src, lut, 0x7650u | (uint32_t)b);
+        else addr = (b ? (src >> (8 * b - 1)) & 0x1feu : (src << 1) & 0x1feu) | lut;
+        uint16_t v;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+        return v;
+    };
+    // bit 31 - 8jj - r of the word is channel r of group jj
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {                       // channels 2i, 2i + 1: bits 7 - 2i and 6 - 2i of the byte
+            const int t = 2 * (3 - jj) + (i < 2 ? 1 : 0), ph = (i & 1) ? 1 : 3;
+            W[jj][i] = entry(ph, t) | (entry(ph - 1, t) << 16);
+        }
 }
 
-// BITS planes; LOOKUP selects the decoder (the byte-permute decoder exists for 3 bits only)
-template <int DT, int BITS, bool LOOKUP>
+template <int DT, int BITS>
 __device__ void ap_pipe_role(const ApParams& p, const FinParams& f, const ApPipeGeom& geo, uint32_t cta, unsigned char* sm) {
-    static_assert(LOOKUP || BITS == 3, "the byte-permute decoder is 3-bit");
+    constexpr bool LOOKUP = BITS > 3;
     constexpr uint32_t kLutRow = 2u << BITS;             // bytes of one row's LUT
     constexpr int NW = 16;                               // consumer warps; warp NW is the producer
     constexpr int NT = (NW + 1) * 32;
@@ -93,7 +107,7 @@ __device__ void ap_pipe_role(const ApParams& p, const FinParams& f, const ApPipe
     const uint32_t bar_empty = bar_full + 64;
     T* sx = reinterpret_cast<T*>(sm + kApPipeHdr);
     float* part = reinterpret_cast<float*>(sm + kApPipeHdr + geo.x_bytes);
-    unsigned char* stage0 = sm + kApPipeHdr + geo.x_bytes + geo.part_bytes;
+    unsigned char* stage0 = sm + kApPipeHdr + geo.x_bytes + geo.part_bytes;      // the byte offsets are multiples of 128
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t nwords = p.K / 32;
@@ -113,7 +127,6 @@ __device__ void ap_pipe_role(const ApParams& p, const FinParams& f, const ApPipe
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (uint32_t i = tid; i < geo.rows_per_cta; i += NT) part[i] = 0.0f;
     __syncthreads();
 
     if (warp == NW) {
@@ -149,191 +162,140 @@ __device__ void ap_pipe_role(const ApParams& p, const FinParams& f, const ApPipe
                 }
             }
         }
-    } else if constexpr (LOOKUP) {
-        // ------------------------------ consumers, lookup decoder -------------------------------
-        pdl_wait();     // weights are already streaming (producer warp); activations come from earlier kernels
-        const T* x = reinterpret_cast<const T*>(p.x);
-        for (uint32_t k = tid; k < p.K; k += 512) sx[k] = x[k];
-        asm volatile("bar.sync 1, 512;" ::: "memory");
-
-        const uint32_t tailE = nwords & 31u, nfull = nwords >> 5;
-        const uint32_t row_in_stage = warp / geo.segs, seg = warp % geo.segs;
-        const bool has_item = row_in_stage < R;
-        const uint32_t wi0 = seg * 128 + lane;            // the lane's words: wi0 + 32 * u, u = 0..3
-        const bool lane_active = has_item && wi0 < nwords;
-
-        for (uint32_t i = 0; i < nst; ++i) {
-            const uint32_t s = i % S;
-            if (!mbar_wait(bar_full + 8 * s, (i / S) & 1u, s_abort, geo.wait_ns)) break;
-            const unsigned char* st = stage0 + (size_t)s * geo.stage_bytes;
-            const uint32_t n = r0 + i * R + row_in_stage;
-            float facc = 0.0f;
-            if (lane_active && n < r1) {
-                const unsigned char* lutrow = st + lut_off + row_in_stage * kLutRow;
-                const uint32_t* rowp = reinterpret_cast<const uint32_t*>(st + (size_t)row_in_stage * rowbytes) + wi0;
-                uint32_t q[4][BITS];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const bool ok = wi0 + 32 * u < nwords;
-#pragma unroll
-                    for (int pl = 0; pl < BITS; ++pl) q[u][pl] = ok ? rowp[32 * u + pl * R * nwords] : 0u;
-                }
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const uint32_t wi = wi0 + 32 * u;
-                    if (wi >= nwords) break;
-                    const uint32_t blk = wi >> 5, t = wi & 31u;
-                    const uint32_t E = (blk == nfull) ? tailE : 32u;
-                    const T* xb = sx + blk * 1024u + 8u * t;
-                    uint4 X[4];
-#pragma unroll
-                    for (int jj = 0; jj < 4; ++jj) X[jj] = *reinterpret_cast<const uint4*>(xb + 8u * E * jj);
-                    ap_lookup_word<DT, BITS>(q[u], lutrow, X, acc);
-                }
-                facc = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_empty + 8 * s);      // the stage (plane words and LUT row) is no longer read
-#pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) facc += __shfl_xor_sync(0xffffffffu, facc, d);
-            if (lane == 0 && has_item && n < r1) {
-                if (geo.segs == 1) part[n - r0] = facc;           // one warp per row: nobody else writes it
-                else atomicAdd(&part[n - r0], facc);              // the K segments of a row meet here
-            }
-        }
     } else {
-        // ------------------------------ consumers, byte-permute decoder -------------------------
+        // ------------------------------ consumers ----------------------------------------------
         pdl_wait();     // weights are already streaming (producer warp); activations come from earlier kernels
         const T* x = reinterpret_cast<const T*>(p.x);
-        for (uint32_t k = tid; k < p.K; k += 512) sx[(k & ~7u) | ap_perm(k & 7u)] = x[k];
-        asm volatile("bar.sync 1, 512;" ::: "memory");
+        // the byte-permute decoder delivers channel pairs (7 - i, 3 - i): its activations are staged in that order
+        for (uint32_t k = tid; k < p.K; k += NW * 32) sx[LOOKUP ? k : ((k & ~7u) | ap_perm(k & 7u))] = x[k];
+        asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
 
-        const uint32_t tailE = nwords & 31u, nfull = nwords >> 5;
-        const uint32_t row_in_stage = warp / geo.segs, seg = warp % geo.segs;
-        const bool has_item = row_in_stage < R;
-        // lane handles words seg*128 + 32*u + lane (u = 0..3): consecutive lanes read consecutive words and
-        // consecutive 16-byte activation groups, so neither shared load has bank conflicts
-        const uint32_t wi0 = seg * 128 + lane;
-        const bool lane_active = has_item && wi0 < nwords;
+        const uint32_t tailE = nwords & 31u;              // words of the row's last, shorter block
+        const uint32_t pair = warp / geo.segs, seg = warp % geo.segs;
+        const uint32_t rowA = 2u * pair, rowB = min(rowA + 1u, R - 1u);   // a stage of one row: its sums are formed twice, used once
+        const bool has_item = rowA < R;
+        // step s of the segment: lane l takes plane word 32 * s + l of both rows, so that consecutive lanes read consecutive words
+        // and consecutive 16-byte activation groups
+        const uint32_t w0 = seg * geo.seg_words;
+        const uint32_t nseg = w0 < nwords ? min(geo.seg_words, nwords - w0) : 0u;
+        const uint32_t full = nseg / 32u;
+        const uint32_t g = lane >> 2;
+        const bool diag = (lane & 3u) == (g >> 1), odd = (g & 1u) != 0u;
+        const uint32_t lutA = smem_u32(sm) + geo.lut_off + warp * 2u * kApLutStride<BITS>;
+        uint32_t* lut_own = reinterpret_cast<uint32_t*>(sm + geo.lut_off + (size_t)warp * 2u * kApLutStride<BITS>);
 
         for (uint32_t i = 0; i < nst; ++i) {
             const uint32_t s = i % S;
             if (!mbar_wait(bar_full + 8 * s, (i / S) & 1u, s_abort, geo.wait_ns)) break;
             const unsigned char* st = stage0 + (size_t)s * geo.stage_bytes;
-            const uint32_t n = r0 + i * R + row_in_stage;
-            float facc = 0.0f;
-            if (lane_active && n < r1) {
-                const uint4 L = *reinterpret_cast<const uint4*>(st + lut_off + row_in_stage * 16);
-                const uint32_t lo01 = __byte_perm(L.x, L.y, 0x6420), lo23 = __byte_perm(L.z, L.w, 0x6420);
-                const uint32_t hi01 = __byte_perm(L.x, L.y, 0x7531), hi23 = __byte_perm(L.z, L.w, 0x7531);
-                const uint32_t* rowp = reinterpret_cast<const uint32_t*>(st + (size_t)row_in_stage * rowbytes) + wi0;
-                uint32_t aw[4], bw[4], cw[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const bool ok = wi0 + 32 * u < nwords;
-                    aw[u] = ok ? rowp[32 * u] : 0u;
-                    bw[u] = ok ? rowp[32 * u + R * nwords] : 0u;
-                    cw[u] = ok ? rowp[32 * u + 2 * R * nwords] : 0u;
+            const uint32_t o = i * R + rowA;                  // first row of the pair, from r0
+            float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+            if (has_item && r0 + o < r1) {
+                const uint32_t* pA = reinterpret_cast<const uint32_t*>(st + (size_t)rowA * rowbytes) + w0 + lane;
+                const uint32_t row_gap = (rowB - rowA) * nwords, plane_gap = R * nwords;
+                LutBytes<3> tA, tB;
+                if constexpr (!LOOKUP) {
+                    const uint4 a = *reinterpret_cast<const uint4*>(st + lut_off + rowA * kLutRow);
+                    const uint4 b = *reinterpret_cast<const uint4*>(st + lut_off + rowB * kLutRow);
+                    tA.fill_pairs(&a.x);
+                    tB.fill_pairs(&b.x);
+                } else {
+                    // the pair's LUT rows to the warp's own, aligned place
+                    __syncwarp();
+                    const uint32_t* lw = reinterpret_cast<const uint32_t*>(st + lut_off + rowA * kLutRow);
+                    constexpr uint32_t half = kLutRow / 4u;
+                    const uint32_t n_lw = rowB > rowA ? 2u * half : half;
+                    for (uint32_t at = lane; at < n_lw; at += 32u) lut_own[at < half ? at : at - half + kApLutStride<BITS> / 4u] = lw[at];
+                    __syncwarp();
                 }
+                // RAGGED: the last step of a segment that is not a whole number of 32 words.  Lanes without one add zero
+                // weights, not table entries that zero activations might turn into NaN.
+                auto step = [&](uint32_t u, auto RAGGED) {
+                    const bool ok = !RAGGED.value || 32u * u + lane < nseg;
+                    const uint32_t blk = (w0 >> 5) + u;
+                    const uint32_t E = RAGGED.value ? tailE : 32u;
+                    uint32_t qA[BITS], qB[BITS];
+                    const uint32_t* at = ok ? pA + 32u * u : pA - lane;        // the segment's first word stands in for one that is not there
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const uint32_t wi = wi0 + 32 * u;
-                    if (wi >= nwords) break;
-                    const uint32_t blk = wi >> 5, t = wi & 31u;
-                    const uint32_t E = (blk == nfull) ? tailE : 32u;
-                    const T* xb = sx + blk * 1024u + 8u * t;
+                    for (int pl = 0; pl < BITS; ++pl) { qA[pl] = at[pl * plane_gap]; qB[pl] = at[pl * plane_gap + row_gap]; }
+                    const T* xb = sx + blk * 1024u + (ok ? 8u * lane : 0u);
                     uint4 X[4];
 #pragma unroll
                     for (int jj = 0; jj < 4; ++jj) X[jj] = *reinterpret_cast<const uint4*>(xb + 8u * E * jj);
-                    const uint32_t a = aw[u];
-                    const uint32_t b = __funnelshift_r(bw[u], bw[u], 1);
-                    const uint32_t c = __funnelshift_r(cw[u], cw[u], 2);
-                    uint32_t V[4];
-                    V[0] = (a & 0x11111111u) | (b & 0x88888888u) | (c & 0x44444444u);
-                    V[0] = __funnelshift_l(V[0], V[0], 2);
-                    V[1] = (a & 0x22222222u) | (b & 0x11111111u) | (c & 0x88888888u);
-                    V[1] = __funnelshift_l(V[1], V[1], 1);
-                    V[2] = (a & 0x44444444u) | (b & 0x22222222u) | (c & 0x11111111u);
-                    V[3] = ((a & 0x88888888u) | (b & 0x44444444u) | (c & 0x22222222u)) >> 1;
-                    uint32_t hacc[4] = {0u, 0u, 0u, 0u};
+                    const uint32_t m = ok ? 0xffffffffu : 0u;
+                    if constexpr (RAGGED.value) {
 #pragma unroll
-                    for (int ph = 0; ph < 4; ++ph) {
-                        const uint32_t v = V[ph];
-                        const uint32_t vh = v >> 16;
-                        const uint32_t l0 = __byte_perm(lo01, lo23, v), h0 = __byte_perm(hi01, hi23, v);
-                        const uint32_t l1 = __byte_perm(lo01, lo23, vh), h1 = __byte_perm(hi01, hi23, vh);
-                        const uint32_t w3 = __byte_perm(l0, h0, 0x5140), w2 = __byte_perm(l0, h0, 0x7362);
-                        const uint32_t w1 = __byte_perm(l1, h1, 0x5140), w0 = __byte_perm(l1, h1, 0x7362);
-                        const uint32_t x3 = (&X[3].x)[ph], x2 = (&X[2].x)[ph], x1 = (&X[1].x)[ph], x0 = (&X[0].x)[ph];
-                        ap_fma<DT>(w3, x3, hacc[3], facc);
-                        ap_fma<DT>(w2, x2, hacc[2], facc);
-                        ap_fma<DT>(w1, x1, hacc[1], facc);
-                        ap_fma<DT>(w0, x0, hacc[0], facc);
+                        for (int jj = 0; jj < 4; ++jj) { X[jj].x &= m; X[jj].y &= m; X[jj].z &= m; X[jj].w &= m; }
                     }
-                    if constexpr (DT == FP16) {
-                        facc += ap_sum2<DT>(hacc[0]) + ap_sum2<DT>(hacc[1]);
-                        facc += ap_sum2<DT>(hacc[2]) + ap_sum2<DT>(hacc[3]);
+                    if constexpr (LOOKUP) {
+                        uint32_t WA[4][4], WB[4][4];
+                        ap_lookup_word<BITS>(qA, lutA, WA);
+                        ap_lookup_word<BITS>(qB, lutA + kApLutStride<BITS>, WB);
+                        if constexpr (RAGGED.value) {
+#pragma unroll
+                            for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) { WA[jj][e] &= m; WB[jj][e] &= m; }
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int jj = 0; jj < 4; ++jj) {
+                            mma_16816<DT>(acc[0], WA[jj][0], WB[jj][0], WA[jj][1], WB[jj][1], X[jj].x, X[jj].y);
+                            mma_16816<DT>(acc[1], WA[jj][2], WB[jj][2], WA[jj][3], WB[jj][3], X[jj].z, X[jj].w);
+                        }
+                    } else {
+                        if constexpr (RAGGED.value) {
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) { tA.lo[e] &= m; tA.hi[e] &= m; tB.lo[e] &= m; tB.hi[e] &= m; }
+                        }
+                        uint32_t VA[4], VB[4];
+                        ap_fields<3>(qA, VA);
+                        ap_fields<3>(qB, VB);
+#pragma unroll
+                        for (int ph = 0; ph < 4; ++ph) {
+                            uint32_t a3, a2, a1, a0, b3, b2, b1, b0;
+                            tA.lookup(VA[ph], a3, a2);
+                            tA.lookup(VA[ph] >> 16, a1, a0);
+                            tB.lookup(VB[ph], b3, b2);
+                            tB.lookup(VB[ph] >> 16, b1, b0);
+                            mma_16816<DT>(acc[0], a3, b3, a2, b2, (&X[3].x)[ph], (&X[2].x)[ph]);
+                            mma_16816<DT>(acc[1], a1, b1, a0, b0, (&X[1].x)[ph], (&X[0].x)[ph]);
+                        }
                     }
-                }
+                };
+#pragma unroll 1
+                for (uint32_t u = 0; u < full; ++u) step(u, IsRagged<false>{});
+                if (full * 32u < nseg) step(full, IsRagged<true>{});
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_empty + 8 * s);      // stage words are in registers
-#pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) facc += __shfl_xor_sync(0xffffffffu, facc, d);
-            if (lane == 0 && has_item && n < r1) {
-                if (geo.segs == 1) part[n - r0] = facc;           // one warp per row: nobody else writes it
-                else atomicAdd(&part[n - r0], facc);              // the K segments of a row meet here
+            if (lane == 0) mbar_arrive(bar_empty + 8 * s);      // the stage (plane words and LUT rows) is no longer read
+            if (diag && has_item && r0 + o < r1) {
+                float* slot = part + ((size_t)o * geo.segs + seg) * 8u + g;
+                slot[0] = odd ? acc[0][1] + acc[1][1] : acc[0][0] + acc[1][0];
+                if (rowA + 1u < R && r0 + o + 1u < r1) slot[geo.segs * 8u] = odd ? acc[0][3] + acc[1][3] : acc[0][2] + acc[1][2];
             }
         }
     }
     if (warp == NW) pdl_wait();     // the producer warp touches the accumulator and y only from here on
-    // fold the CTA's rows: four consecutive outputs per thread; y is read before the barrier so that the
-    // load overlaps the last warps' work
+    // fold the CTA's rows: a row's slots in order, one output per thread; y is read before the barrier so that the load
+    // overlaps the last warps' work
     T* y = reinterpret_cast<T*>(f.y);
     const uint32_t nrows = r1 - r0;
-    const bool yvec = geo.direct && (nrows & 3u) == 0u && (r0 & 3u) == 0u &&
-                      (reinterpret_cast<uintptr_t>(f.y) & (4u * sizeof(T) - 1u)) == 0u;
-    float y0[4] = {0.f, 0.f, 0.f, 0.f};
-    const bool pre = yvec && 4u * (uint32_t)tid < nrows;
-    if (pre) {
-        const uint2 raw = *reinterpret_cast<const uint2*>(y + r0 + 4u * tid);
-        const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) y0[i] = Tr<DT>::to_f(e[i]);
-    }
+    float y0 = 0.0f;
+    if (geo.direct && (uint32_t)tid < nrows) y0 = Tr<DT>::to_f(y[r0 + tid]);
     __syncthreads();
     if (*s_abort && tid == 0) raise_error(f.err, 1u);
-    if (geo.direct) {
-        if (!*s_abort) {            // an unfinished launch leaves y alone
-            if (yvec) {
-                for (uint32_t i = 4u * tid; i < nrows; i += 4u * NT) {
-                    const float4 v = *reinterpret_cast<const float4*>(part + i);
-                    float o[4];
-                    if (pre && i == 4u * (uint32_t)tid) { o[0] = y0[0]; o[1] = y0[1]; o[2] = y0[2]; o[3] = y0[3]; }
-                    else {
-                        const uint2 raw = *reinterpret_cast<const uint2*>(y + r0 + i);
-                        const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) o[q] = Tr<DT>::to_f(e[q]);
-                    }
-                    o[0] += v.x; o[1] += v.y; o[2] += v.z; o[3] += v.w;
-                    uint2 raw;
-                    T* e = reinterpret_cast<T*>(&raw);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) e[q] = Tr<DT>::from_f(o[q]);
-                    *reinterpret_cast<uint2*>(y + r0 + i) = raw;
-                }
-            } else {
-                for (uint32_t i = tid; i < nrows; i += NT)
-                    y[r0 + i] = Tr<DT>::from_f(Tr<DT>::to_f(y[r0 + i]) + part[i]);
-            }
-        }
-        return;
+    if (geo.direct && *s_abort) return;      // an unfinished launch leaves y alone
+    for (uint32_t i = tid; i < nrows; i += NT) {
+        const float4* slots = reinterpret_cast<const float4*>(part + (size_t)i * geo.segs * 8u);
+        float v = 0.0f;
+        for (uint32_t e = 0; e < 2u * geo.segs; ++e) { const float4 q = slots[e]; v += (q.x + q.y) + (q.z + q.w); }
+        if (geo.direct) y[r0 + i] = Tr<DT>::from_f((i == (uint32_t)tid ? y0 : Tr<DT>::to_f(y[r0 + i])) + v);
+        else __stcg(f.acc + r0 + i, *s_abort ? 0.0f : v);
     }
-    // fused launch: the sums go to the accumulator (this CTA is their only GEMV writer) and the CTA arrives on its
+    if (geo.direct) return;
+    // fused launch: the sums went to the accumulator (this CTA is their only GEMV writer) and the CTA arrives on its
     // tile even after a failed wait, so that the workspace stays consistent
-    for (uint32_t i = tid; i < nrows; i += NT) __stcg(f.acc + r0 + i, part[i]);
     arrive_and_finalize<DT>(f, cta, cta + 1, s_flag, NT);
 }
 

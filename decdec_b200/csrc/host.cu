@@ -385,11 +385,12 @@ int run_anyprec(Config* c, const void* x, void* y, const int32_t* qw, uint32_t p
     uint32_t budget = gemv_sm_budget(c, true);
     if (c) {
         // many compensation thread blocks (the launch is bound by the host link): the GEMV runs in the SMs they leave
-        // free and takes over the rest as they retire, which it does more evenly in thread blocks a third the size
+        // free and takes over the rest as they retire, which it does more evenly in thread blocks half the size (eight fused
+        // 4-bit launches of two 8B blocks at k_chunk 8: 220 / 214 / 228 us for one, two and three)
         DecParams dg;
         memset(&dg, 0, sizeof(dg));
         dec_geometry(c, true, 1u << 20, &dg);
-        if (dg.n_cta > device_sms() / 4 + 3) budget *= env_u32("DECDEC_AP_FUSED_SPLIT", 3);
+        if (dg.n_cta > device_sms() / 4 + 3) budget *= env_u32("DECDEC_AP_FUSED_SPLIT", 2);
     }
     const bool pipe = env_u32("DECDEC_AP_PIPE", 1) && anyprec_pipe_geometry(N, K, g.bits, &pgeo, budget, c == nullptr);
     if (pipe) tile_units = cdiv(pgeo.rows_per_cta, 32);

@@ -42,20 +42,13 @@ cudaError_t launch_anyprec(int dt, const ApParams& g, const DecParams& d, const 
     return fast3 ? go<BF16, true>(g, d, f, s) : go<BF16, false>(g, d, f, s);
 }
 
-template <int DT, int BITS, bool LOOKUP>
+template <int DT, int BITS>
 __global__ void __launch_bounds__(kApPipeThreads, 1)
 k_anyprec_pipe(const __grid_constant__ ApParams g, const __grid_constant__ DecParams d, const __grid_constant__ FinParams f,
                const __grid_constant__ ApPipeGeom geo) {
-    extern __shared__ __align__(128) unsigned char sm[];
+    extern __shared__ __align__(512) unsigned char sm[];     // the warps' LUT rows are aligned to kApLutStride
     if (blockIdx.x < d.n_cta) dec_role<DT>(d, f, blockIdx.x, sm);
-    else ap_pipe_role<DT, BITS, LOOKUP>(g, f, geo, blockIdx.x - d.n_cta, sm);
-}
-
-// Which decoder a 3-bit launch takes: the register-table one unless DECDEC_AP3_DECODER=lookup.
-static bool ap_lookup_decoder(uint32_t bits) {
-    if (bits != 3) return true;
-    const char* v = getenv("DECDEC_AP3_DECODER");
-    return v && *v == 'l';
+    else ap_pipe_role<DT, BITS>(g, f, geo, blockIdx.x - d.n_cta, sm);
 }
 
 // Stage geometry of the pipelined kernel (3 to 8 bits); false if the shape is not eligible.  A CTA's rows are a whole
@@ -64,34 +57,51 @@ static bool ap_lookup_decoder(uint32_t bits) {
 // instead of 96 of 64).
 bool anyprec_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, ApPipeGeom* geo, uint32_t sm_budget, bool gemv_only) {
     if (bits < 3 || bits > 8 || K % 128u || K > 32768u || N == 0) return false;
-    const bool lookup = ap_lookup_decoder(bits);
     const uint32_t rowbytes = K / 8;
     const uint32_t per_row = bits * rowbytes + (2u << bits);      // plane words and the LUT row
-    geo->segs = (K + 4095) / 4096;
-    uint32_t R = 16 / geo->segs;
-    if (R == 0) return false;
-    while (R & (R - 1)) R &= R - 1;                      // largest power of two <= 16 / segs
-    geo->lookup = lookup ? 1u : 0u;
     geo->x_bytes = (K * 2 + 127u) & ~127u;
     if (sm_budget == 0) sm_budget = 1;
     uint32_t rows = (N + sm_budget - 1) / sm_budget;
     const uint32_t gran = gemv_only ? 16u : 32u;
     rows = ((rows + gran - 1) / gran) * gran;
     geo->rows_per_cta = rows;
-    geo->part_bytes = (rows * 4u + 127u) & ~127u;
-    const uint32_t fixed = kApPipeHdr + geo->x_bytes + geo->part_bytes;
-    if (fixed >= 227u * 1024u) return false;
-    const uint32_t budget = 227 * 1024 - fixed;
-    // wide rows: fewer rows per stage until two stages fit (some consumer warps then have no work item)
-    while (R > 1 && 2u * ((R * per_row + 127u) & ~127u) > budget) R >>= 1;
-    geo->rows_per_stage = R;
-    geo->stage_bytes = (R * per_row + 127u) & ~127u;
-    uint32_t smax = budget / geo->stage_bytes;
-    if (smax > 8) smax = 8;
-    if (smax < 2) return false;
-    const uint32_t nst = rows / R;
-    geo->stages = nst < smax ? nst : smax;
-    geo->smem_bytes = fixed + geo->stages * geo->stage_bytes;
+    const uint32_t lut_stride = bits <= 7 ? kApLutStride<7> : kApLutStride<8>;
+    const uint32_t lut_bytes = bits > 3 ? 16u * 2u * lut_stride + lut_stride : 0u;       // 16 warps, and room for the alignment
+    // Cut of a stage over the 16 warps: rows in pairs, a row's 1024-channel blocks in `segs` segments.  A stage costs its
+    // warps the blocks of a segment plus about 0.8 of a block for the wait, the tables and the sums; long segments spread
+    // that best, short ones fill the warps when the CTA has few rows (and leave room for two stages of wide rows).
+    const uint32_t nblk = (K + 1023u) / 1024u;
+    uint32_t best = 0xffffffffu;
+    for (uint32_t want = 1; want <= 16; ++want) {
+        const uint32_t blocks = (nblk + want - 1) / want, segs = (nblk + blocks - 1) / blocks;
+        const uint32_t part = (rows * segs * 32u + 127u) & ~127u;
+        const uint32_t fixed = kApPipeHdr + geo->x_bytes + part + lut_bytes;
+        if (segs > 16 || fixed >= 227u * 1024u) continue;
+        const uint32_t budget = 227u * 1024u - fixed;
+        uint32_t R = 2u * (16u / segs);
+        while (R & (R - 1)) R &= R - 1;
+        while (R > 2 && R / 2 >= rows) R >>= 1;
+        // wide rows: fewer rows per stage until two stages fit (some consumer warps then have no work item)
+        while (R > 1 && 2u * ((R * per_row + 127u) & ~127u) > budget) R >>= 1;
+        const uint32_t stage = (R * per_row + 127u) & ~127u;
+        if (2u * stage > budget) continue;
+        const uint32_t nst = (rows + R - 1) / R;
+        const uint32_t cost = nst * (10u * blocks + 8u);
+        if (cost >= best) continue;
+        best = cost;
+        uint32_t smax = budget / stage;
+        if (smax > 8) smax = 8;
+        geo->segs = segs;
+        geo->seg_words = 32u * blocks;
+        geo->part_bytes = part;
+        geo->rows_per_stage = R;
+        geo->stage_bytes = stage;
+        geo->stages = nst < smax ? nst : smax;
+        const uint32_t end = kApPipeHdr + geo->x_bytes + part + geo->stages * stage;
+        geo->lut_off = (end + lut_stride - 1u) & ~(lut_stride - 1u);
+        geo->smem_bytes = bits > 3 ? geo->lut_off + 16u * 2u * lut_stride : end;
+    }
+    if (best == 0xffffffffu) return false;
     geo->direct = 0;        // set by the caller
     {
         const char* w = getenv("DECDEC_PIPE_WAIT_NS");
@@ -101,13 +111,13 @@ bool anyprec_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, ApPipeGeom* ge
     return true;
 }
 
-template <int DT, int BITS, bool LOOKUP>
+template <int DT, int BITS>
 static cudaError_t go_pipe(const ApParams& g, const DecParams& d, const FinParams& f, const ApPipeGeom& geo, cudaStream_t s) {
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_anyprec_pipe<DT, BITS, LOOKUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaError_t e = cudaFuncSetAttribute(k_anyprec_pipe<DT, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
@@ -124,18 +134,18 @@ static cudaError_t go_pipe(const ApParams& g, const DecParams& d, const FinParam
     attr[0].val.programmaticStreamSerializationAllowed = (e && *e == '0') ? 0 : 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_anyprec_pipe<DT, BITS, LOOKUP>, g, d, f, geo);
+    return cudaLaunchKernelEx(&cfg, k_anyprec_pipe<DT, BITS>, g, d, f, geo);
 }
 
 template <int DT>
 static cudaError_t pipe_by_bits(const ApParams& g, const DecParams& d, const FinParams& f, const ApPipeGeom& geo, cudaStream_t s) {
     switch (g.bits) {
-        case 3: return geo.lookup ? go_pipe<DT, 3, true>(g, d, f, geo, s) : go_pipe<DT, 3, false>(g, d, f, geo, s);
-        case 4: return go_pipe<DT, 4, true>(g, d, f, geo, s);
-        case 5: return go_pipe<DT, 5, true>(g, d, f, geo, s);
-        case 6: return go_pipe<DT, 6, true>(g, d, f, geo, s);
-        case 7: return go_pipe<DT, 7, true>(g, d, f, geo, s);
-        case 8: return go_pipe<DT, 8, true>(g, d, f, geo, s);
+        case 3: return go_pipe<DT, 3>(g, d, f, geo, s);
+        case 4: return go_pipe<DT, 4>(g, d, f, geo, s);
+        case 5: return go_pipe<DT, 5>(g, d, f, geo, s);
+        case 6: return go_pipe<DT, 6>(g, d, f, geo, s);
+        case 7: return go_pipe<DT, 7>(g, d, f, geo, s);
+        case 8: return go_pipe<DT, 8>(g, d, f, geo, s);
         default: return cudaErrorInvalidValue;
     }
 }

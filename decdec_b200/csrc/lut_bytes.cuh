@@ -4,21 +4,30 @@
 
 namespace dd {
 
-// 4-bit fields from up to four plane words: field t (bits 4t..4t+3) of result ph holds, most significant plane
-// first, the bits that planes P[0..B-1] carry at position 4t + ph.
+template <bool V> struct IsRagged { static constexpr bool value = V; };     // compile-time argument of a generic lambda
+
+// Up to four plane words, regrouped: nibble position 4t of result ph, rotated left by B - 1 - ph, starts the field of the bits
+// that planes P[0..B-1] carry at position 4t + ph, most significant plane first.
 template <int B>
-__device__ __forceinline__ void ap_fields(const uint32_t* P, uint32_t (&V)[4]) {
+__device__ __forceinline__ void ap_merge(const uint32_t* P, uint32_t (&M)[4]) {
     uint32_t R[B];
 #pragma unroll
     for (int i = 0; i < B; ++i) R[i] = i ? __funnelshift_r(P[i], P[i], i) : P[0];
 #pragma unroll
     for (int ph = 0; ph < 4; ++ph) {
-        uint32_t m = 0u;
+        M[ph] = 0u;
 #pragma unroll
-        for (int i = 0; i < B; ++i) m |= R[i] & (0x11111111u << ((ph - i) & 3));
-        const int rot = (B - 1 - ph) & 31;
-        V[ph] = rot ? __funnelshift_l(m, m, rot) : m;
+        for (int i = 0; i < B; ++i) M[ph] |= R[i] & (0x11111111u << ((ph - i) & 3));
     }
+}
+__device__ __forceinline__ uint32_t rotate_left(uint32_t v, int by) { return (by & 31) ? __funnelshift_l(v, v, by & 31) : v; }
+
+// 4-bit fields: field t (bits 4t..4t+3) of result ph holds the code bits of position 4t + ph.
+template <int B>
+__device__ __forceinline__ void ap_fields(const uint32_t* P, uint32_t (&V)[4]) {
+    ap_merge<B>(P, V);
+#pragma unroll
+    for (int ph = 0; ph < 4; ++ph) V[ph] = rotate_left(V[ph], B - 1 - ph);
 }
 
 // A table of 2^BITS 16-bit values in registers, split into low and high bytes so that one byte permute looks up the low (or

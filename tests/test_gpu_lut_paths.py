@@ -1,4 +1,5 @@
-"""Edges of the table-lookup kernels on the GPU: ragged layers (binary-coded), pair tables (SqueezeLLM), vector dequantizers.
+"""Edges of the table-lookup kernels on the GPU: ragged layers (binary-coded), pair tables (SqueezeLLM), row
+pairs (any-precision), vector dequantizers.
 
 Oracle: the dense weights of the packed tensors in float64.  Tolerances of the GEMVs: products and sums are fp32, and the output is rounded once; with y = 0 before the call the error of an output is at most
 half an ulp of it (2^-11 or 2^-8 of its size in fp16 and bf16) plus the fp32 sum's, K * 2^-24 of the sum of magnitudes, which
@@ -8,6 +9,7 @@ import numpy as np
 import pytest
 import torch
 
+from oracle import formats
 from tests import problems as P
 
 pytestmark = pytest.mark.gpu
@@ -85,6 +87,40 @@ def test_sqllm_values_that_are_not_finite_stay_in_their_column(ops, bits):
     rest = np.ones(N, bool)
     rest[[5, 70, 133]] = False
     _assert_sums(torch.from_numpy(got[rest]), L["w_hat"][rest], x, "fp16")
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("N,K,bits", [
+    (1, 128, 3), (17, 128, 4), (33, 2048, 3), (33, 2048, 4), (47, 2176, 3), (47, 2176, 8), (300, 6272, 3), (31, 6272, 6),
+    (3, 32768, 3), (3, 32768, 8), (2999, 1152, 3), (2999, 1152, 5), (2999, 1152, 7),
+])
+def test_anyprec_row_pairs(ops, dtype, N, K, bits):
+    L = P.lut_layer(N, K, bits, seed=N + K + bits, dtype=dtype, real=False)
+    x = P.make_activation(K, seed=8, dtype=dtype)
+    held = torch.zeros(K + 1, dtype=x.dtype, device="cuda")
+    for xd in (x.cuda(), held[1:].copy_(x.reshape(-1)).view(1, 1, K)):        # aligned, and one element into a buffer
+        y = torch.zeros(1, 1, N, dtype=P.TORCH_DT[dtype], device="cuda")
+        ops.anyprec_gemv(xd, y, L["qweight"].cuda(), L["lut"].cuda(), bits)
+        _assert_sums(y, L["w_hat"], x, dtype)
+
+
+@pytest.mark.parametrize("bits", [3, 4])
+def test_anyprec_values_that_are_not_finite_stay_in_their_row(ops, bits):
+    """Lanes without a plane word (K = 1152: a tail block of four words) add nothing, whatever their row's table holds."""
+    N, K = 64, 1152
+    L = P.lut_layer(N, K, bits, seed=10, real=False)
+    codes, lut = L["codes"].copy(), L["lut"].clone()
+    codes[codes == 0] = 1
+    lut[:, 0] = float("inf")                              # an entry that no weight uses
+    lut[9, 1] = float("nan")
+    x = P.make_activation(K, seed=8)
+    y = torch.zeros(1, 1, N, dtype=torch.float16, device="cuda")
+    ops.anyprec_gemv(x.cuda(), y, torch.from_numpy(formats.anyprec_pack(codes, bits).copy()).cuda(), lut.cuda(), bits)
+    got = P.to_np(y).reshape(-1)
+    w_hat = np.take_along_axis(P.to_np(lut), codes.astype(np.int64), 1)
+    assert np.isnan(got[9])
+    rest = np.arange(N) != 9
+    _assert_sums(torch.from_numpy(got[rest]), w_hat[rest], x, "fp16")
 
 
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
