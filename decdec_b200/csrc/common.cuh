@@ -73,6 +73,11 @@ struct DecParams {
     uint32_t fused_select;     // 1: select rows from x; 0: rows are given in sel_rows
 };
 
+// quotient of an index that is almost always below 2^32: the 64-bit division costs about five times the 32-bit one
+__device__ __forceinline__ uint32_t quotient(size_t v, uint32_t by) {
+    return (v >> 32) == 0u ? (uint32_t)v / by : (uint32_t)(v / by);
+}
+
 __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
     uint4 v;
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThreads) ap_dequant_kernel(const uint32_t* __
     const size_t plane_stride = total;
     constexpr int BH = BITS < 4 ? BITS : 4, BL = BITS - BH;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t n = (uint32_t)(idx / nwords), wi = (uint32_t)(idx % nwords);
+        const uint32_t n = quotient(idx, nwords), wi = (uint32_t)(idx - (size_t)n * nwords);
         uint32_t q[BITS];
 #pragma unroll
         for (int pl = 0; pl < BITS; ++pl) q[pl] = ldg_stream(qweight + pl * plane_stride + idx);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kThreads) ap_dequant_kernel(const uint32_t* __
                                   entry(3, 2 * b) | (entry(2, 2 * b) << 16), entry(1, 2 * b) | (entry(0, 2 * b) << 16));
         }
 #pragma unroll
-        for (int b = 0; b < 4; ++b) *reinterpret_cast<uint4*>(o + 8u * E * (3 - b)) = v[b];
+        for (int b = 0; b < 4; ++b) __stcs(reinterpret_cast<uint4*>(o + 8u * E * (3 - b)), v[b]);
     }
 }
 

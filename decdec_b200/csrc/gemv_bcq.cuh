@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kThreads) bcq_dequant_vec_kernel(const uint32_
     const uint32_t nquad = N / 4;
     const size_t total = (size_t)(K / 32) * nquad;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t kw = (uint32_t)(idx / nquad), n = 4u * (uint32_t)(idx % nquad);
+        const uint32_t kw = quotient(idx, nquad), n = 4u * (uint32_t)(idx - (size_t)kw * nquad);
         const uint32_t g = (kw * 32u) / group;
         uint4 w[BITS];
         uint2 ar[BITS];
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kThreads) bcq_dequant_vec_kernel(const uint32_
                     uint2 o;
                     o.x = t < 2 ? __byte_perm(e01[0], e01[1], sel) : __byte_perm(e23[0], e23[1], sel);
                     o.y = t < 2 ? __byte_perm(e01[2], e01[3], sel) : __byte_perm(e23[2], e23[3], sel);
-                    *reinterpret_cast<uint2*>(dst + (size_t)(16 * h + 4 * t + ph) * N) = o;
+                    __stcs(reinterpret_cast<uint2*>(dst + (size_t)(16 * h + 4 * t + ph) * N), o);
                 }
             }
         }
