@@ -167,7 +167,8 @@ __device__ __forceinline__ void pipe_load_x8(const void* xbase, uint32_t k0, boo
     }
 }
 
-template <int DT, int BITS>
+// RAGGED: the layer has a partial last stage or K slice (see above); the others do without the checks
+template <int DT, int BITS, bool RAGGED>
 __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const PipeGeom& geo, const PipeMaps& maps,
                               uint32_t cta, unsigned char* sm) {
     using T = typename Tr<DT>::T;
@@ -284,6 +285,7 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
         const bool swapAB = (tA & 4) != 0;                  // after the swap X = group r, Y = group r + 4, r = tA & 3
         const uint32_t r4 = tA & 3;
         const uint32_t n_out = blk * 32 + ((j & 4) ? 16 : 0) + 4 * r4 + (j & 3);
+        float* acc_lane = f.acc + (size_t)st0 * kPipeStageN + n_out;
         bool pending = false;
         unsigned long long p_old = 0, p_mine = 0;
         unsigned long long* p_word = nullptr;
@@ -293,7 +295,7 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
         pdl_wait();     // weights are already streaming (producer warp); activations come from earlier kernels
         if (builder && !*s_abort) {
             float xv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (kbase + koff < p.K) pipe_load_x8<DT>(p.x, kbase + koff, xvec, xv);     // K is a multiple of 32
+            if (!RAGGED || kbase + koff < p.K) pipe_load_x8<DT>(p.x, kbase + koff, xvec, xv);     // K is a multiple of 32
             float lo[8], hi[4];
 #pragma unroll
             for (int e = 0; e < 8; ++e)
@@ -368,12 +370,12 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
                 const float keep = (j & 1) ? y2[1] : y2[0];
                 y1 = keep + __shfl_sync(0xffffffffu, send, p1);
             }
-            const uint32_t n = (st0 + i) * kPipeStageN + n_out;
-            if (!geo.packed) {
-                if (n < p.N) atomicAdd(f.acc + n, y1);
+            if (RAGGED || !geo.packed) {
+                if (!RAGGED || (st0 + i) * kPipeStageN + n_out < p.N) atomicAdd(acc_lane + i * kPipeStageN, y1);
             } else {
                 // the previous stage's atomic has long returned: settle it, then send this stage's
                 if (pending) finish_packed<DT>(p_old, p_mine, geo.arrivals, p_word, p_y, p_y0);
+                const uint32_t n = (st0 + i) * kPipeStageN + n_out;
                 p_word = reinterpret_cast<unsigned long long*>(f.acc) + n;
                 p_y = reinterpret_cast<T*>(f.y) + n;
                 p_y0 = Tr<DT>::to_f(*p_y);

@@ -38,7 +38,8 @@ k_bcq_pipe(const __grid_constant__ BcqParams g, const __grid_constant__ DecParam
         if (geo.packed) dec_role_packed<DT>(d, f, blockIdx.x, sm, geo.arrivals);
         else dec_role<DT>(d, f, blockIdx.x, sm);
     } else {
-        bcq_pipe_role<DT, BITS>(g, f, geo, maps, blockIdx.x - d.n_cta, sm);
+        if (g.N % kPipeStageN || g.K % kBcqSlice) bcq_pipe_role<DT, BITS, true>(g, f, geo, maps, blockIdx.x - d.n_cta, sm);
+        else bcq_pipe_role<DT, BITS, false>(g, f, geo, maps, blockIdx.x - d.n_cta, sm);
     }
 }
 
