@@ -5,7 +5,7 @@
 // through registers: a producer thread moves a tile of [16 k-rows x bits planes] x 128 outputs (+ the
 // alpha and q_bias rows that go with them) per stage from HBM to shared memory with three tiled TMA
 // copies (cp.async.bulk.tensor.2d, completion counted on an mbarrier), several stages ahead of the
-// consumer warps (three groups of eight, taking stages round-robin).  HBM latency is then covered by
+// consumer warps (three groups of eight, taking stages round-robin: stage_ring.h).  HBM latency is then covered by
 // bytes in flight (about 29 KB per stage, up to 5 stages per SM) instead of by occupancy.  The tile
 // lands densely (512-byte lines); the lanes of a warp read it in a skewed order (k-row j reads the
 // 16-byte groups (j + c) mod 8 and +4), so every 128-bit shared load of a quarter warp touches eight
@@ -39,6 +39,7 @@
 #pragma once
 #include "common.cuh"
 #include "gemv_bcq.cuh"
+#include "stage_ring.h"
 #include <cuda.h>
 #include "dec_role.cuh"
 
@@ -52,6 +53,8 @@ constexpr uint32_t kPipeSuspendNs = 20000u;      // a poll may sleep this long i
 
 struct PipeGeom {
     uint32_t stages;         // pipeline depth S
+    uint32_t fulls;          // `full` barriers (stage_ring.h)
+    uint32_t inv_stages, inv_fulls;      // ring_inverse of the two
     uint32_t stage_bytes;    // bytes of one stage in shared memory
     uint32_t w_bytes;        // weight part of a stage
     uint32_t a_bytes;        // alpha part of a stage
@@ -136,8 +139,9 @@ __device__ __forceinline__ void lds4f(const unsigned char* base, uint32_t elem, 
 // Shared memory.  The 64 KB of tables start at the first shared-window address that is a multiple of
 // 64 KB, so that a lookup address {entry byte, slot offset} is complete after ONE byte-permute (bits
 // 16.. of the address come from two constant bytes); the pipeline stages fill the space before and after:
-//   [header 256 B: row sums, flags, 8 full + 8 empty barriers][stages ...][tables @ 64 KB multiple][stages ...]
-constexpr int kPipeHdr = 256;
+//   [header 384 B: row sums, flags, up to 16 full + 8 empty barriers][stages ...][tables @ 64 KB multiple][stages ...]
+constexpr int kPipeHdr = 384;
+constexpr uint32_t kPipeSlots = 8, kPipeFulls = 16;          // at most
 constexpr uint32_t kPipeTblOffAssumed = 65536 - 1024;   // dynamic shared memory normally starts 1 KB into the window
 
 // stages that fit before the tables when these start `tbl_off` bytes into dynamic shared memory
@@ -181,7 +185,7 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
     volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(sm + 64);
     unsigned* s_flag = reinterpret_cast<unsigned*>(sm + 64 + 4);
     const uint32_t bar_full = smem_u32(sm + 80);
-    const uint32_t bar_empty = bar_full + 64;
+    const uint32_t bar_empty = bar_full + 8 * kPipeFulls;
     const uint32_t n_before = pipe_stages_before(tbl_off, geo.stage_bytes);
     auto stage_ptr = [&](uint32_t s) -> unsigned char* {
         return s < n_before ? sm + kPipeHdr + (size_t)s * geo.stage_bytes
@@ -206,10 +210,8 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
         const uint32_t after = S > n_before ? S - n_before : 0u;
         const bool bad = tbl_off + kBcqTableBytes + after * geo.stage_bytes > dyn || (tbl_off & 127u);
         *s_abort = bad ? 2u : 0u;
-        for (uint32_t s = 0; s < S; ++s) {
-            mbar_init(bar_full + 8 * s, 1);
-            mbar_init(bar_empty + 8 * s, 8);
-        }
+        for (uint32_t b = 0; b < geo.fulls; ++b) mbar_init(bar_full + 8 * b, 1);
+        for (uint32_t s = 0; s < S; ++s) mbar_init(bar_empty + 8 * s, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -224,15 +226,15 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
             tma_prefetch_desc(&maps.a);
             tma_prefetch_desc(&maps.b);
             for (uint32_t i = 0; i < n_issue; ++i) {
-                const uint32_t s = i % S, use = i / S;
-                if (use > 0) {
+                const uint32_t s = ring_place(i, S, geo.inv_stages);
+                if (i >= S) {
                     // A slot frees only after the consumers have passed their own wait for the previous kernel, which
                     // may itself be waiting for another GPU: the bounded wait must not run during that time.  Every
                     // slot is full at this point, so waiting for the dependency here delays no copy.
-                    if (use == 1 && s == 0) pdl_wait();
-                    if (!mbar_wait(bar_empty + 8 * s, (use - 1) & 1u, s_abort, geo.wait_ns)) break;
+                    if (i == S) pdl_wait();
+                    if (!mbar_wait(bar_empty + 8 * s, ring_parity(i - S, geo.inv_stages), s_abort, geo.wait_ns)) break;
                 }
-                const uint32_t full = bar_full + 8 * s;
+                const uint32_t full = bar_full + 8 * ring_place(i, geo.fulls, geo.inv_fulls);
                 mbar_expect_tx(full, tx);
                 const uint32_t n0 = (st0 + i) * kPipeStageN;
                 const uint32_t dst = smem_u32(stage_ptr(s));
@@ -246,7 +248,7 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
                 const uint32_t first = issued > S ? issued - S : 0;
                 for (uint32_t i = first; i < issued; ++i) {
                     volatile uint32_t never = 0;
-                    mbar_wait(bar_full + 8 * (i % S), (i / S) & 1u, &never, 1000000000u);
+                    mbar_wait(bar_full + 8 * ring_place(i, geo.fulls, geo.inv_fulls), ring_parity(i, geo.inv_fulls), &never, 1000000000u);
                 }
             }
         }
@@ -319,8 +321,9 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
         const float sx = rowsum[krow];
 
         for (uint32_t i = grp; i < nst && !*s_abort; i += kPipeGroups) {
-            const uint32_t s = i % S;
-            if (!mbar_wait(bar_full + 8 * s, (i / S) & 1u, s_abort, geo.wait_ns)) break;
+            const uint32_t s = ring_place(i, S, geo.inv_stages);
+            const uint32_t full = bar_full + 8 * ring_place(i, geo.fulls, geo.inv_fulls);
+            if (!mbar_wait(full, ring_parity(i, geo.inv_fulls), s_abort, geo.wait_ns)) break;
             const unsigned char* st = stage_ptr(s);
             const unsigned char* wl = st + krow * (BITS * kPipeLine);
             const unsigned char* al = st + geo.w_bytes + (g * BITS) * (kPipeStageN * ESZ);

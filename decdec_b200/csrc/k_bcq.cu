@@ -154,13 +154,16 @@ bool bcq_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, uint32_t group, in
     const uint32_t n_before = pipe_stages_before(kPipeTblOffAssumed, geo->stage_bytes);
     const uint32_t room_after = 227 * 1024 - (kPipeTblOffAssumed + kBcqTableBytes);
     uint32_t smax = n_before + room_after / geo->stage_bytes;
-    if (smax > 8) smax = 8;
+    if (smax > kPipeSlots) smax = kPipeSlots;
     if (smax < 2) return false;
     const uint32_t nst_total = (N + kPipeStageN - 1) / kPipeStageN;
     // one CTA per SM; tiles sized so that the grid is at most one wave
     uint32_t per1 = sm_budget / n_kslices; if (per1 == 0) per1 = 1;
     geo->tile_stages = (nst_total + per1 - 1) / per1;
     geo->stages = geo->tile_stages < smax ? geo->tile_stages : smax;
+    geo->fulls = ring_full_barriers(geo->stages, kPipeGroups);
+    geo->inv_stages = ring_inverse(geo->stages);
+    geo->inv_fulls = ring_inverse(geo->fulls);
     const uint32_t after = geo->stages > n_before ? geo->stages - n_before : 0;
     geo->smem_bytes = kPipeTblOffAssumed + kBcqTableBytes + after * geo->stage_bytes;
     if (geo->smem_bytes < (uint32_t)DecSmem::kBytes) geo->smem_bytes = DecSmem::kBytes;
