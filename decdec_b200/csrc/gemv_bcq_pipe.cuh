@@ -225,6 +225,8 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
             tma_prefetch_desc(&maps.w);
             tma_prefetch_desc(&maps.a);
             tma_prefetch_desc(&maps.b);
+            // ragged layers are ordered like plain launches: their weights may come from the kernel before
+            if (RAGGED) pdl_wait();
             for (uint32_t i = 0; i < n_issue; ++i) {
                 const uint32_t s = ring_place(i, S, geo.inv_stages);
                 if (i >= S) {

@@ -153,3 +153,34 @@ def test_lutgemm_dequant_forms(ops, dtype, bits, N, K, group):
         total = total + torch.from_numpy(bit[:, p].astype(np.float32) * 2 - 1) * alpha.float()[gidx, p]
     expected = total.to(P.TORCH_DT[dtype]) + bias[gidx]
     assert torch.equal(out.view(torch.int16), expected.view(torch.int16))
+
+
+def _overlapped_producer(ops):
+    """A GEMV that lets the next launch start before its own outputs are written: [28672] values of about 0.02."""
+    N, K = 28672, 4096
+    g = torch.Generator(device="cuda").manual_seed(2)
+    qw = torch.randint(-2**31, 2**31 - 1, (K // 32, 3, N), dtype=torch.int32, device="cuda", generator=g)
+    alpha = (torch.rand((K // 128, 3, N), device="cuda", generator=g) * 0.01).half()
+    bias = torch.zeros((K // 128, N), device="cuda").half()
+    x = (torch.randn((1, 1, K), device="cuda", generator=g) * 0.02).half()
+    y = torch.zeros(1, 1, N, device="cuda").half()
+
+    def produce():
+        y.zero_()
+        ops.lutgemm_gemv(x, y, qw, alpha, bias, 3, 128)
+    return y.view(-1), produce
+
+
+def test_ragged_scales_may_come_from_the_launch_before(ops):
+    N, K, bits, group = 136, 544, 4, 32
+    made, produce = _overlapped_producer(ops)
+    alpha = made[: K // group * bits * N].view(K // group, bits, N)
+    L = P.random_bcq_layer(N, K, bits, group, seed=21)
+    x, qw, bias = P.make_activation(K, seed=22).cuda(), L["qweight"].cuda(), L["q_bias"].cuda()
+    produce()
+    w_hat = formats.bcq_dequant(L["qweight"].numpy(), P.to_np(alpha), P.to_np(L["q_bias"]), group)
+    for _ in range(20):
+        y = torch.zeros(1, 1, N, device="cuda").half()
+        produce()
+        ops.lutgemm_gemv(x, y, qw, alpha, bias, bits, group)
+        _assert_sums(y, w_hat, x, "fp16")
