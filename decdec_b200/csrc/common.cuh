@@ -236,18 +236,17 @@ __device__ __forceinline__ void finalize_span(const FinParams& f, uint32_t n0, u
 // Must be called by all threads of the CTA, after all its reductions into the accumulators were issued.
 // `nthreads` = number of threads of the CTA that take part (threads beyond it must have exited; the
 // first warp always takes part).  The tickets of up to 32 tiles are taken by one warp in parallel, so a
-// CTA that covers many tiles pays one atomic round trip, not one per tile.  `arrivals` = what this CTA counts for on each
-// of the tiles: a role whose CTAs share a tile unevenly counts the work they did, so that the sum per tile is fixed.
+// CTA that covers many tiles pays one atomic round trip, not one per tile.
 template <int DT>
 __device__ __forceinline__ void arrive_and_finalize(const FinParams& f, uint32_t t0, uint32_t t1, unsigned* s_flag,
-                                                    uint32_t nthreads = kThreads, uint32_t arrivals = 1u) {
+                                                    uint32_t nthreads = kThreads) {
     __threadfence();
     __syncthreads();
     for (uint32_t tb = t0; tb < t1; tb += 32u) {
         if (threadIdx.x < 32u) {
             const uint32_t t = tb + threadIdx.x;
             bool last = false;
-            if (t < t1) last = (atomicAdd(&f.tickets[t], arrivals) + arrivals == f.expected);
+            if (t < t1) last = (atomicAdd(&f.tickets[t], 1u) + 1u == f.expected);
             const unsigned m = __ballot_sync(0xffffffffu, last);
             if (threadIdx.x == 0) *s_flag = m;
         }

@@ -12,10 +12,12 @@
 // spread to the quad's other columns: a tile whose tables hold such a value is summed with fp32 multiply-adds instead.
 //
 // Split of the work.  The (64-column tile, 32-channel group) units are one line that is cut evenly over the thread blocks, so
-// every SM gets the same share whatever N and K are (whole tiles would leave 25 % of the SMs idle at 28672 columns).  A tile
-// that one thread block covers alone is added to y directly; the parts of the others meet in the fp32 accumulator, and a part
-// arrives on the tile's ticket with the number of groups it covered, so that K / 32 arrivals complete a tile however it was
-// cut (common.cuh).  Tables are built from the weights' LUT, and the first words loaded, before the wait for the previous kernel.
+// every SM gets the same share whatever N and K are (whole tiles would leave 25 % of the SMs idle at 28672 columns).  A thread
+// block has at most two cut parts, its first and its last: a cut part's sums go to a place of their own in the workspace, and
+// the part takes a ticket of the tile with the number of groups it covered; whoever brings the tickets to K / 32 adds the
+// parts in the order of their channels, so that equal calls give equal bits.  The sums of a tile are then added to y, or, beside a
+// compensation role, stored in the accumulator with one arrival on the tile (common.cuh).
+// Tables are built from the weights' LUT, and the first words loaded, before the wait for the previous kernel.
 //
 // Measured, 4 bits, fp16, us per launch in a graph: 28672 x 4096 35 -> 24.2, and the eight linears of two 8B blocks 187 -> 125,
 // against one lookup, one conversion and one fp32 multiply-add per weight.  What is left over the wavefronts (20 000 of 43 000
@@ -122,6 +124,26 @@ __device__ __forceinline__ void sq_pair_sums(const uint32_t* __restrict__ col, u
     if (g < g1) consume(g, w0);
 }
 
+// Sums of the 64 columns of a tile whose parts lie in the workspace, in the order of the channels: v of thread tid < 64.
+// Thread block c covers units [units * c / n_cta, units * (c + 1) / n_cta); its first part is at slot 2 c, a last part that starts
+// with a tile of its own at slot 2 c + 1.
+__device__ __forceinline__ float sq_pair_join(const SqParams& p, uint32_t tile, uint32_t groups, uint64_t units) {
+    const uint64_t u0 = (uint64_t)tile * groups;
+    const uint32_t c0 = (uint32_t)(((u0 + 1) * p.n_cta - 1) / units), c1 = (uint32_t)(((u0 + groups) * p.n_cta - 1) / units);
+    const float* at = p.parts + (size_t)c0 * 2u * kSqTileN + (units * c0 / p.n_cta == u0 ? 0u : kSqTileN) + threadIdx.x;
+    float v = __ldcg(at);
+    at = p.parts + threadIdx.x;
+    constexpr uint32_t U = 4;                               // loads in flight
+    for (uint32_t c = c0 + 1; c <= c1; c += U) {
+        float q[U];
+#pragma unroll
+        for (uint32_t i = 0; i < U; ++i) q[i] = c + i <= c1 ? __ldcg(at + (size_t)(c + i) * 2u * kSqTileN) : 0.0f;
+#pragma unroll
+        for (uint32_t i = 0; i < U; ++i) if (c + i <= c1) v += q[i];
+    }
+    return v;
+}
+
 template <int DT, int BITS>
 __device__ void sq_pair_role(const SqParams& p, const FinParams& f, uint32_t cta, unsigned char* sm) {
     using T = typename Tr<DT>::T;
@@ -138,7 +160,8 @@ __device__ void sq_pair_role(const SqParams& p, const FinParams& f, uint32_t cta
     T* y = reinterpret_cast<T*>(f.y);
 
     const uint64_t units = (uint64_t)f.n_tiles * groups;
-    uint64_t u = units * cta / p.n_cta;
+    const uint64_t ubegin = units * cta / p.n_cta;
+    uint64_t u = ubegin;
     const uint64_t uend = units * (cta + 1) / p.n_cta;
     bool waited = false;
     pdl_trigger();
@@ -201,15 +224,37 @@ __device__ void sq_pair_role(const SqParams& p, const FinParams& f, uint32_t cta
             *reinterpret_cast<float2*>(part + warp * kSqTileN + 2u * lane) = make_float2(acc[0][0], acc[0][1]);
         }
         __syncthreads();
-        const bool whole = p.direct && g1 - g0 == groups;
-        if (tid < kSqTileN && n0 + tid < p.N) {
-            float v = 0.0f;
+        const bool whole = g1 - g0 == groups, mine = tid < kSqTileN && n0 + tid < p.N;
+        float v = 0.0f;
+        if (tid < kSqTileN) {
 #pragma unroll
             for (uint32_t w = 0; w < NW; ++w) v += part[w * kSqTileN + tid];
-            if (whole) y[n0 + tid] = Tr<DT>::from_f(Tr<DT>::to_f(y[n0 + tid]) + v);
-            else atomicAdd(&f.acc[n0 + tid], v);
         }
-        if (!whole) arrive_and_finalize<DT>(f, tile, tile + 1, s_flag, kSqPairThreads, g1 - g0);
+        bool joined = whole;
+        if (!whole) {
+            if (tid < kSqTileN) __stcg(p.parts + (2u * cta + (u == ubegin ? 0u : 1u)) * kSqTileN + tid, v);
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) {
+                const bool last = atomicAdd(p.part_tickets + tile, g1 - g0) + (g1 - g0) == groups;
+                if (last) p.part_tickets[tile] = 0u;
+                *s_flag = last;
+            }
+            __syncthreads();
+            joined = *s_flag != 0u;
+            if (joined && tid < kSqTileN) {
+                __threadfence();
+                v = sq_pair_join(p, tile, groups, units);
+            }
+        }
+        if (joined) {
+            if (p.direct) {
+                if (mine) y[n0 + tid] = Tr<DT>::from_f(Tr<DT>::to_f(y[n0 + tid]) + v);
+            } else {
+                if (mine) __stcg(f.acc + n0 + tid, v);
+                arrive_and_finalize<DT>(f, tile, tile + 1, s_flag, kSqPairThreads);
+            }
+        }
         u = (uint64_t)tile * groups + g1;
     }
     if (!waited) pdl_wait();

@@ -49,6 +49,8 @@ int fail(int code, const char* fmt, ...) {
 
 constexpr uint32_t kAccCap = 1u << 18;      // outputs per call supported by the accumulator
 constexpr uint32_t kTicketCap = 1u << 13;
+constexpr uint32_t kSqMaxCta = 320;         // thread blocks of a pair-table launch: room for the sums of their cut parts
+constexpr uint32_t kPartCap = kSqMaxCta * 2u * kSqTileN;
 
 struct Workspace {
     float* acc = nullptr;
@@ -56,6 +58,7 @@ struct Workspace {
     unsigned* err = nullptr;          // device-visible address of the error word (mapped pinned host memory)
     volatile unsigned* err_host = nullptr;   // the same word as the host sees it: read before every launch, no copy needed
     float* acc2 = nullptr;            // second half of the accumulator allocation (compensation sums)
+    float* parts = nullptr;           // behind it: sums that are written before they are read, never cleared
 };
 
 std::mutex g_mu;
@@ -78,10 +81,11 @@ int check_ws(const Workspace& w) {
 // Allocates and clears one workspace (never called while a stream of the device is capturing).
 static int alloc_workspace(Workspace* out) {
     Workspace w;
-    if (cudaMalloc(&w.acc, 2 * kAccCap * sizeof(float)) != cudaSuccess) return fail(DECDEC_E_NOMEM, "cudaMalloc(accumulator) failed");
+    if (cudaMalloc(&w.acc, (2 * kAccCap + kPartCap) * sizeof(float)) != cudaSuccess) return fail(DECDEC_E_NOMEM, "cudaMalloc(accumulator) failed");
     if (cudaMalloc(&w.tickets, (kTicketCap + 4) * sizeof(unsigned)) != cudaSuccess) { cudaFree(w.acc); return fail(DECDEC_E_NOMEM, "cudaMalloc(tickets) failed"); }
     DD_CUDA(cudaMemset(w.acc, 0, 2 * kAccCap * sizeof(float)));
     w.acc2 = w.acc + kAccCap;
+    w.parts = w.acc + 2 * kAccCap;
     DD_CUDA(cudaMemset(w.tickets, 0, (kTicketCap + 4) * sizeof(unsigned)));
     {
         // the error word lives in mapped pinned host memory: a kernel that gives up stores into it, and the
@@ -429,17 +433,20 @@ int run_sqllm(Config* c, const void* x, void* y, const int32_t* qw, const void* 
     g.lut = lut;
     g.x = x;
     g.K = K; g.N = N; g.bits = (uint32_t)bits;
-    // 16-bit layers with an even number of outputs take the pair tables; a tile counts K / 32 arrivals there
+    // 16-bit layers with an even number of outputs take the pair tables
     const bool pair = env_u32("DECDEC_SQ_PAIR", 1) && sqllm_pair_eligible(qw, lut, N, K, g.bits, dtype);
     FinParams f;
-    if (int r = setup_fin(&f, ws, y, N, pair ? kSqTileN / 32u : 1u, pair ? K / 32u : 1u)) return r;
+    if (int r = setup_fin(&f, ws, y, N, pair ? kSqTileN / 32u : 1u, 1)) return r;
     g.n_cta = f.n_tiles;
     if (pair) {
         // two thread blocks per SM hide each other's table builds, but none is made for less than sixteen groups
         const uint64_t units = (uint64_t)f.n_tiles * (K / 32u);
         uint64_t n = 2u * gemv_sm_budget(c, true);
         if (n > (units + 15u) / 16u) n = (units + 15u) / 16u;
+        if (n > kSqMaxCta) n = kSqMaxCta;
         g.n_cta = (uint32_t)n;
+        g.parts = ws.parts;
+        g.part_tickets = ws.tickets + f.n_tiles;     // tiles are twice as wide as the capacity was made for
     }
     DecParams d;
     memset(&d, 0, sizeof(d));

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 import torch
 
-from oracle import formats
+from oracle import formats, forward
 from tests import problems as P
 
 pytestmark = pytest.mark.gpu
@@ -62,7 +62,7 @@ def test_lutgemm_ragged_layers(ops, dtype, N, K, bits, group):
     (66, 1024),         # a tile of two columns
     (63, 256),          # odd: general kernel
     (190, 8192),        # tiles cut over several thread blocks
-    (9600, 768),        # more tiles than thread blocks: whole tiles and cut ones
+    (9600, 768),        # many tiles of few groups
 ])
 def test_sqllm_pair_tables(ops, dtype, bits, N, K):
     L = P.lut_layer(N, K, bits, seed=N + K + bits, dtype=dtype, fmt="sqllm", real=False)
@@ -153,6 +153,47 @@ def test_lutgemm_dequant_forms(ops, dtype, bits, N, K, group):
         total = total + torch.from_numpy(bit[:, p].astype(np.float32) * 2 - 1) * alpha.float()[gidx, p]
     expected = total.to(P.TORCH_DT[dtype]) + bias[gidx]
     assert torch.equal(out.view(torch.int16), expected.view(torch.int16))
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("N,K,bits,n_tb", [
+    (2050, 320, 4, 0),         # two columns in the last tile
+    (4096, 4096, 3, 0),        # every tile in several parts
+    (19200, 2336, 4, 0),       # whole tiles and cut ones in one thread block
+    (2056, 2400, 4, 16),       # beside a compensation, eight columns in the last tile
+    (9536, 2336, 4, 148),
+])
+def test_sqllm_parts_of_a_tile(ops, dtype, N, K, bits, n_tb):
+    """Sums of parts meet in a fixed order: repeated calls give the same bits, on top of outputs that are not zero."""
+    L = P.lut_layer(N, K, bits, seed=N + K, dtype=dtype, fmt="sqllm", real=False)
+    x = P.make_activation(K, seed=7, dtype=dtype)
+    y0 = (torch.randn(1, 1, N, generator=torch.Generator().manual_seed(3)) * 2).to(P.TORCH_DT[dtype])
+    qw, lut, xd = L["qweight"].cuda(), L["lut"].cuda(), x.cuda()
+    ref = L["w_hat"] @ P.to_np(x).reshape(-1) + P.to_np(y0).reshape(-1)
+    mags = np.abs(L["w_hat"]) @ np.abs(P.to_np(x).reshape(-1)) + np.abs(P.to_np(y0).reshape(-1))
+    outs = []
+    for _ in range(8):
+        y = y0.clone().cuda()
+        ops.sqllm_gemv(xd, y, qw, lut, bits)
+        outs.append(y)
+    assert all(torch.equal(y, outs[0]) for y in outs)
+    if n_tb:
+        cs, rs = P.random_residual(N, K, seed=5, dtype=dtype)
+        thr = P.make_thresholds(K, dtype, n_calib=32)
+        k = 4 * K // 1024
+        rows, acts = torch.zeros(k, dtype=torch.int32, device="cuda"), torch.zeros(k, dtype=P.TORCH_DT[dtype], device="cuda")
+        ctx = ops.create_dec_context(n_tb, rows, acts)
+        cfg = ops.create_dec_config(ctx, 4, cs, rs, thr)
+        exp_rows, exp_acts, _ = P.expected_selection(x, thr, 4, dtype)
+        delta = forward.dec_delta(P.to_np(x), exp_rows, cs.numpy(), P.to_np(rs), exp_acts)
+        for _ in range(2):                               # the second call finds the workspace as the first left it
+            y = y0.clone().cuda()
+            ops.dec_sqllm(cfg, xd, y, qw, lut, bits)
+            bound = HALF_ULP[dtype] * np.abs(ref + delta) + K * 2.0 ** -24 * (mags + np.abs(delta)) + 2.0 ** -24
+            assert (np.abs(P.to_np(y).reshape(-1) - ref - delta) <= bound).all()
+        ops.destroy_dec_config(cfg)
+    bound = HALF_ULP[dtype] * np.abs(ref) + K * 2.0 ** -24 * mags + 2.0 ** -24
+    assert (np.abs(P.to_np(outs[0]).reshape(-1) - ref) <= bound).all()
 
 
 def _overlapped_producer(ops):
