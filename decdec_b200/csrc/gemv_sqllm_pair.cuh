@@ -11,18 +11,18 @@
 // fp32 multiply-adds would need eight, and eight conversions.  A zero of B times an infinite or NaN weight would
 // spread to the quad's other columns: a tile whose tables hold such a value is summed with fp32 multiply-adds instead.
 //
-// Split of the work.  The (64-column tile, 32-channel group) units are one line that is cut evenly over the thread blocks, so
-// every SM gets the same share whatever N and K are (whole tiles would leave 25 % of the SMs idle at 28672 columns).  A thread
-// block has at most two cut parts, its first and its last: a cut part's sums go to a place of their own in the workspace, and
+// Split of the work.  The (64-column tile, 32-channel group) units are one line that is cut evenly over the thread blocks.  Where it
+// pays their number is a multiple of the tiles' (host.cu:sqllm_pair_blocks), so that a thread block has one part and one table to
+// build.  A thread block has at most two cut parts, its first and its last: a cut part's sums go to a place of their own in the workspace, and
 // the part takes a ticket of the tile with the number of groups it covered; whoever brings the tickets to K / 32 adds the
 // parts in the order of their channels, so that equal calls give equal bits.  The sums of a tile are then added to y, or, beside a
 // compensation role, stored in the accumulator with one arrival on the tile (common.cuh).
 // Tables are built from the weights' LUT, and the first words loaded, before the wait for the previous kernel.
 //
 // Measured, 4 bits, fp16, us per launch in a graph: 28672 x 4096 35 -> 24.2, and the eight linears of two 8B blocks 187 -> 125,
-// against one lookup, one conversion and one fp32 multiply-add per weight.  What is left over the wavefronts (20 000 of 43 000
-// cycles) is the latency of a part's start (tables, first words) and end (sums of the warps): two thread blocks per SM overlap
-// them (180 us with one), cutting only at eighths of a tile, for fewer parts, does not help (127 us).
+// against one lookup, one conversion and one fp32 multiply-add per weight; the cut at tiles brought 24.4 -> 22.8 and 125 -> 100.  What
+// is left over the wavefronts (20 000 cycles of a 28672 x 4096 launch) is the latency of a part's start (tables, first words) and end
+// (sums of the warps): two thread blocks per SM overlap them (180 us with one).
 #pragma once
 #include "common.cuh"
 #include "gemv_sqllm.cuh"

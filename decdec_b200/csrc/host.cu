@@ -420,6 +420,36 @@ int run_anyprec(Config* c, const void* x, void* y, const int32_t* qw, uint32_t p
     return 0;
 }
 
+// Thread blocks of a pair-table launch: two fit an SM, beside the compensation's.  Either every tile is cut into `m` equal parts (or not at
+// all), so that a thread block has one table to build, or, where the tiles don't divide the SMs well, the whole line of (tile,
+// group) units is cut evenly and most thread blocks have two.  The estimates, in 1/100 us, are fitted to launches of 8 to 500 tiles
+// and 16 to 896 groups at 4 bits: a start and an end, a join of the parts, and the groups of a thread block at the rate of one or
+// two on an SM.  Measured, even cut of the line -> this rule, 4 bits, us: 512 x 1792 6.7 -> 4.1 (general kernel 5.0), 4096 x 4096 9.8 -> 6.8,
+// 6144 x 4096 11.0 -> 7.8, 4096 x 14336 15.5 -> 12.9, 14336 x 1024 9.9 -> 5.0, 28672 x 4096 24.4 -> 22.8, and beside 48 compensation
+// thread blocks at k_chunk 8 42.1 -> 26.1; 10240 x 8192 stays with the line (18.6, whole tiles 20.4).
+uint32_t sqllm_pair_blocks(const Config* c, uint32_t n_tiles, uint32_t groups) {
+    const uint32_t sms = device_sms();
+    uint32_t slots = 2u * sms;
+    if (c) {
+        DecParams d;
+        memset(&d, 0, sizeof(d));
+        dec_geometry(c, true, 1u << 20, &d);
+        slots = d.n_cta < sms ? slots - d.n_cta : sms;
+    }
+    if (slots > kSqMaxCta) slots = kSqMaxCta;
+    const uint64_t units = (uint64_t)n_tiles * groups;
+    const uint32_t line = (uint32_t)(units < slots ? units : slots);
+    uint64_t best = 670u + 91u * (units / line) / 10u;
+    uint32_t blocks = line;
+    for (uint32_t m = 1; m == 1u || (m * n_tiles <= slots && 12u * m <= groups); ++m) {
+        const uint32_t n = m * n_tiles;
+        const uint64_t rounds = cdiv(n, slots);
+        const uint64_t t = (m > 1u ? 460u : 260u) + rounds * cdiv(groups, m) * (n <= sms ? 50u : 75u) / 10u;
+        if (t <= best) { best = t; blocks = n; }
+    }
+    return blocks;
+}
+
 int run_sqllm(Config* c, const void* x, void* y, const int32_t* qw, const void* lut, uint32_t N, uint32_t K, int bits,
               int dtype, cudaStream_t s) {
     if (int r = check_gemv_common(x, y, qw, N, K, dtype)) return r;
@@ -439,12 +469,7 @@ int run_sqllm(Config* c, const void* x, void* y, const int32_t* qw, const void* 
     if (int r = setup_fin(&f, ws, y, N, pair ? kSqTileN / 32u : 1u, 1)) return r;
     g.n_cta = f.n_tiles;
     if (pair) {
-        // two thread blocks per SM hide each other's table builds, but none is made for less than sixteen groups
-        const uint64_t units = (uint64_t)f.n_tiles * (K / 32u);
-        uint64_t n = 2u * gemv_sm_budget(c, true);
-        if (n > (units + 15u) / 16u) n = (units + 15u) / 16u;
-        if (n > kSqMaxCta) n = kSqMaxCta;
-        g.n_cta = (uint32_t)n;
+        g.n_cta = sqllm_pair_blocks(c, f.n_tiles, K / 32u);
         g.parts = ws.parts;
         g.part_tickets = ws.tickets + f.n_tiles;     // tiles are twice as wide as the capacity was made for
     }
