@@ -22,6 +22,7 @@ struct SqParams {
     uint32_t K, N, bits;
     uint32_t n_cta;            // ceil(N / 32); pair tables: thread blocks the work is cut over
     uint32_t direct;
+    uint32_t part_groups;      // pair tables: 32-channel groups of the longest part
     float* parts;              // pair tables: sums of cut parts, [2 * n_cta][64]
     unsigned* part_tickets;    // and the tickets of the tiles that have them
 };

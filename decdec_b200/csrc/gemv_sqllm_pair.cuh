@@ -34,9 +34,14 @@ constexpr uint32_t kSqTileN = 64;                         // columns per tile = 
 constexpr uint32_t kSqPartBytes = (kSqPairThreads / 32) * kSqTileN * 4;
 
 __host__ __device__ inline uint32_t sq_pair_table_bytes(uint32_t bits) { return 256u << (2u * bits); }
-// tables, activations of one segment, partial sums of the warps, flag
-__host__ __device__ inline uint32_t sq_pair_smem(uint32_t K, uint32_t bits) {
-    return sq_pair_table_bytes(bits) + ((K * 2u + 15u) & ~15u) + kSqPartBytes + 16u;
+// tables, activations of the longest part, partial sums of the warps, flag
+__host__ __device__ inline uint32_t sq_pair_smem(uint32_t part_groups, uint32_t bits) {
+    return sq_pair_table_bytes(bits) + part_groups * 64u + kSqPartBytes + 16u;
+}
+// groups of the longest part when `units` are cut over n_cta thread blocks
+inline uint32_t sq_pair_part_groups(uint64_t units, uint32_t n_cta, uint32_t groups) {
+    const uint64_t share = (units + n_cta - 1u) / n_cta;
+    return share < groups ? (uint32_t)share : groups;
 }
 
 __device__ __forceinline__ uint2 ldg_stream(const uint2* p) {
@@ -152,7 +157,7 @@ __device__ void sq_pair_role(const SqParams& p, const FinParams& f, uint32_t cta
     constexpr uint32_t NW = kSqPairThreads / 32;
     const uint32_t tbytes = sq_pair_table_bytes(BITS);
     T* sx = reinterpret_cast<T*>(sm + tbytes);
-    float* part = reinterpret_cast<float*>(sm + tbytes + ((p.K * 2u + 15u) & ~15u));
+    float* part = reinterpret_cast<float*>(sm + tbytes + p.part_groups * 64u);
     unsigned* s_flag = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(part) + kSqPartBytes);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t groups = p.K / 32;

@@ -464,12 +464,13 @@ int run_sqllm(Config* c, const void* x, void* y, const int32_t* qw, const void* 
     g.x = x;
     g.K = K; g.N = N; g.bits = (uint32_t)bits;
     // 16-bit layers with an even number of outputs take the pair tables
-    const bool pair = env_u32("DECDEC_SQ_PAIR", 1) && sqllm_pair_eligible(qw, lut, N, K, g.bits, dtype);
+    const bool pair = env_u32("DECDEC_SQ_PAIR", 1) && sqllm_pair_eligible(qw, lut, N, dtype);
     FinParams f;
     if (int r = setup_fin(&f, ws, y, N, pair ? kSqTileN / 32u : 1u, 1)) return r;
     g.n_cta = f.n_tiles;
     if (pair) {
         g.n_cta = sqllm_pair_blocks(c, f.n_tiles, K / 32u);
+        g.part_groups = sq_pair_part_groups((uint64_t)f.n_tiles * (K / 32u), g.n_cta, K / 32u);
         g.parts = ws.parts;
         g.part_tickets = ws.tickets + f.n_tiles;     // tiles are twice as wide as the capacity was made for
     }

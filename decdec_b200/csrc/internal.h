@@ -20,7 +20,7 @@ cudaError_t launch_anyprec(int dt, const ApParams& g, const DecParams& d, const 
 bool anyprec_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, ApPipeGeom* geo, uint32_t sm_budget = 148, bool gemv_only = false);
 cudaError_t launch_anyprec_pipe(int dt, const ApParams& g, const DecParams& d, const FinParams& f, const ApPipeGeom& geo, cudaStream_t s);
 cudaError_t launch_sqllm(int dt, const SqParams& g, const DecParams& d, const FinParams& f, cudaStream_t s);
-bool sqllm_pair_eligible(const void* qweight, const void* lut, uint32_t N, uint32_t K, uint32_t bits, int dt);
+bool sqllm_pair_eligible(const void* qweight, const void* lut, uint32_t N, int dt);
 cudaError_t launch_sqllm_pair(int dt, const SqParams& g, const DecParams& d, const FinParams& f, cudaStream_t s);
 cudaError_t launch_ap_dequant(int dt, const uint32_t* qweight, const void* lut, void* out, uint32_t N, uint32_t K,
                               uint32_t bits, cudaStream_t s);

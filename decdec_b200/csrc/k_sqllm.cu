@@ -51,7 +51,7 @@ k_sqllm_pair(const __grid_constant__ SqParams g, const __grid_constant__ DecPara
 
 template <int DT, int BITS, bool DEC>
 static cudaError_t go_pair_dec(const SqParams& g, const DecParams& d, const FinParams& f, cudaStream_t s) {
-    size_t smem = sq_pair_smem(g.K, g.bits);
+    size_t smem = sq_pair_smem(g.part_groups, g.bits);
     if (DEC && smem < (size_t)DecSmem::kBytes) smem = DecSmem::kBytes;
     static bool configured[64] = {};
     int dev = 0;
@@ -81,12 +81,13 @@ static cudaError_t go_pair(const SqParams& g, const DecParams& d, const FinParam
     return d.n_cta ? go_pair_dec<DT, BITS, true>(g, d, f, s) : go_pair_dec<DT, BITS, false>(g, d, f, s);
 }
 
-bool sqllm_pair_eligible(const void* qweight, const void* lut, uint32_t N, uint32_t K, uint32_t bits, int dt) {
+// (shared memory: the 50 000 channels that run_sqllm takes need 166 KB in one part)
+bool sqllm_pair_eligible(const void* qweight, const void* lut, uint32_t N, int dt) {
     int dev = 0, reserved = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess) { cudaGetLastError(); return false; }
     return (uint32_t)reserved == kSqTableBase && dt != FP32 && N % 2u == 0u && (reinterpret_cast<uintptr_t>(qweight) & 7u) == 0u &&
-           (reinterpret_cast<uintptr_t>(lut) & 15u) == 0u && sq_pair_smem(K, bits) <= 227u * 1024u;
+           (reinterpret_cast<uintptr_t>(lut) & 15u) == 0u;
 }
 
 cudaError_t launch_sqllm_pair(int dt, const SqParams& g, const DecParams& d, const FinParams& f, cudaStream_t s) {
