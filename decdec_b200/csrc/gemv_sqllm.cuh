@@ -8,8 +8,8 @@
 // A CTA owns 32 output columns for the whole of K: lane = column (128-byte coalesced word rows),
 // warp = K slice.  The column LUTs sit in shared memory as fp32 [code][column], so lane l always hits
 // bank l.  Sums are fp32; the eight K slices are combined in shared memory, so no cross-CTA
-// reduction is needed.  General form: fp32 layers, odd numbers of outputs and unaligned tensors; 16-bit layers take the
-// pair tables of gemv_sqllm_pair.cuh.
+// reduction is needed.  General form: fp32 layers, odd numbers of outputs, unaligned tensors and small layers (host.cu:
+// run_sqllm); the others take the pair tables of gemv_sqllm_pair.cuh.
 #pragma once
 #include "common.cuh"
 

@@ -17,11 +17,11 @@
 // the part takes a ticket of the tile with the number of groups it covered; whoever brings the tickets to K / 32 adds the
 // parts in the order of their channels, so that equal calls give equal bits.  The sums of a tile are then added to y, or, beside a
 // compensation role, stored in the accumulator with one arrival on the tile (common.cuh).
-// Tables are built from the weights' LUT, and the first words loaded, before the wait for the previous kernel.
+// The launch may become resident while the previous kernel of the stream drains, but reads nothing before that one has
+// completed: codes and centroids may come from it.  (Tables and first words ahead of the wait were worth 1.0 to 1.6 us per launch.)
 //
-// Measured, 4 bits, fp16, us per launch in a graph: 28672 x 4096 35 -> 24.2, and the eight linears of two 8B blocks 187 -> 125,
-// against one lookup, one conversion and one fp32 multiply-add per weight; the cut at tiles brought 24.4 -> 22.8 and 125 -> 100.  What
-// is left over the wavefronts (20 000 cycles of a 28672 x 4096 launch) is the latency of a part's start (tables, first words) and end
+// Measured, 4 bits, fp16, us per launch in a graph, against one lookup, one conversion and one fp32 multiply-add per weight: 28672 x 4096
+// 35.6 -> 25.1, 4096 x 14336 32.4 -> 14.3, and the eight linears of two 8B blocks 187 -> 115.6 (125 with the even cut).  What is left over the wavefronts (20 000 cycles of a 28672 x 4096 launch) is the latency of a part's start (tables, first words) and end
 // (sums of the warps): two thread blocks per SM overlap them (180 us with one).
 #pragma once
 #include "common.cuh"
@@ -168,12 +168,12 @@ __device__ void sq_pair_role(const SqParams& p, const FinParams& f, uint32_t cta
     const uint64_t ubegin = units * cta / p.n_cta;
     uint64_t u = ubegin;
     const uint64_t uend = units * (cta + 1) / p.n_cta;
-    bool waited = false;
     pdl_trigger();
     if ((uint32_t)__cvta_generic_to_shared(sm) != kSqTableBase) {     // not the layout the launch was made for: nothing is computed
         if (tid == 0) raise_error(f.err, 2u);
         return;
     }
+    pdl_wait();
     while (u < uend) {
         const uint32_t tile = (uint32_t)(u / groups), g0 = (uint32_t)(u % groups);
         const uint32_t g1 = (uint32_t)(uend - (uint64_t)tile * groups < groups ? uend - (uint64_t)tile * groups : groups);
@@ -211,7 +211,6 @@ __device__ void sq_pair_role(const SqParams& p, const FinParams& f, uint32_t cta
                     dst[(hi * NC + lo) * 64u] = __byte_perm(pr[lo / 2], hv, (lo & 1u) ? 0x5432u : 0x5410u);
             }
         }
-        if (!waited) { pdl_wait(); waited = true; }         // activations, outputs and the workspace come from earlier kernels
         for (uint32_t k = tid; k < (g1 - g0) * 32u; k += kSqPairThreads) sx[k] = x[g0 * 32u + k];
         const bool finite = !__syncthreads_or(bad);
 
@@ -262,7 +261,6 @@ __device__ void sq_pair_role(const SqParams& p, const FinParams& f, uint32_t cta
         }
         u = (uint64_t)tile * groups + g1;
     }
-    if (!waited) pdl_wait();
 }
 
 }  // namespace dd

@@ -463,8 +463,11 @@ int run_sqllm(Config* c, const void* x, void* y, const int32_t* qw, const void* 
     g.lut = lut;
     g.x = x;
     g.K = K; g.N = N; g.bits = (uint32_t)bits;
-    // 16-bit layers with an even number of outputs take the pair tables
-    const bool pair = env_u32("DECDEC_SQ_PAIR", 1) && sqllm_pair_eligible(qw, lut, N, dtype);
+    // 16-bit layers with an even number of outputs take the pair tables.  Small ones of few channels don't: a table is then used
+    // too little (us, 4 bits, general kernel / pair tables: 3072 x 1024 4.0 / 4.9, 1000 x 2176 5.0 / 6.3, 2048 x 2048 6.1 / 6.7,
+    // 8192 x 1024 5.0 / 5.4; 768 x 4096 7.8 / 7.1, 14336 x 1024 8.2 / 6.2)
+    const bool small = K <= 2304u && (uint64_t)cdiv(N, kSqTileN) * (K / 32u) <= 4096u;
+    const bool pair = env_u32("DECDEC_SQ_PAIR", 1) && !small && sqllm_pair_eligible(qw, lut, N, dtype);
     FinParams f;
     if (int r = setup_fin(&f, ws, y, N, pair ? kSqTileN / 32u : 1u, 1)) return r;
     g.n_cta = f.n_tiles;

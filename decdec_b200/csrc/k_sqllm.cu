@@ -61,7 +61,7 @@ static cudaError_t go_pair_dec(const SqParams& g, const DecParams& d, const FinP
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
-    // programmatic dependent launch: the pair tables are built while the previous kernel of the stream drains
+    // programmatic dependent launch: the thread blocks become resident while the previous kernel of the stream drains
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(d.n_cta + g.n_cta);
     cfg.blockDim = dim3(kSqPairThreads);
@@ -70,7 +70,7 @@ static cudaError_t go_pair_dec(const SqParams& g, const DecParams& d, const FinP
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     const char* e = getenv("DECDEC_PDL");
-    attr[0].val.programmaticStreamSerializationAllowed = (e && *e == '0') ? 0 : 1;
+    attr[0].val.programmaticStreamSerializationAllowed = (e && (*e == '0' || (*e == '1' && DEC))) ? 0 : 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_sqllm_pair<DT, BITS, DEC>, g, d, f);

@@ -63,6 +63,9 @@ def test_lutgemm_ragged_layers(ops, dtype, N, K, bits, group):
     (63, 256),          # odd: general kernel
     (190, 8192),        # tiles cut over several thread blocks
     (9600, 768),        # many tiles of few groups
+    (9600, 1024),       # small layers above take the general kernel
+    (2, 2336),
+    (66, 2400),
 ])
 def test_sqllm_pair_tables(ops, dtype, bits, N, K):
     L = P.lut_layer(N, K, bits, seed=N + K + bits, dtype=dtype, fmt="sqllm", real=False)
@@ -73,9 +76,10 @@ def test_sqllm_pair_tables(ops, dtype, bits, N, K):
         _assert_sums(y, L["w_hat"], x, dtype)
 
 
+@pytest.mark.parametrize("K", [1024, 2400])      # general kernel, pair tables
 @pytest.mark.parametrize("bits", [3, 4])
-def test_sqllm_values_that_are_not_finite_stay_in_their_column(ops, bits):
-    N, K = 256, 1024
+def test_sqllm_values_that_are_not_finite_stay_in_their_column(ops, bits, K):
+    N = 256
     L = P.lut_layer(N, K, bits, seed=9, fmt="sqllm", real=False)
     lut = L["lut"].clone()
     lut[5, 1], lut[70, 2], lut[133, 0] = float("inf"), float("nan"), float("-inf")
@@ -224,4 +228,19 @@ def test_ragged_scales_may_come_from_the_launch_before(ops):
         y = torch.zeros(1, 1, N, device="cuda").half()
         produce()
         ops.lutgemm_gemv(x, y, qw, alpha, bias, bits, group)
+        _assert_sums(y, w_hat, x, "fp16")
+
+
+def test_sqllm_tables_may_come_from_the_launch_before(ops):
+    N, K, bits = 1792, 2336, 4
+    made, produce = _overlapped_producer(ops)
+    lut = made[: N * 2 ** bits].view(N, 2 ** bits)
+    L = P.lut_layer(N, K, bits, seed=23, fmt="sqllm", real=False)
+    x, qw = P.make_activation(K, seed=24).cuda(), L["qweight"].cuda()
+    produce()
+    w_hat = formats.lut_dequant(P.to_np(lut), L["codes"])
+    for _ in range(20):
+        y = torch.zeros(1, 1, N, device="cuda").half()
+        produce()
+        ops.sqllm_gemv(x, y, qw, lut, bits)
         _assert_sums(y, w_hat, x, "fp16")
