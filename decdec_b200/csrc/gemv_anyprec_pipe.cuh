@@ -42,7 +42,7 @@ struct ApPipeGeom {
     uint32_t x_bytes;          // staged activations (rounded to 128)
     uint32_t rows_per_cta;     // multiple of R
     uint32_t part_bytes;       // partial sums of the CTA: fp32 [row][segment][8]
-    uint32_t lut_off;          // where the lookup decoder's warps keep their LUT rows (aligned to kApLutStride)
+    uint32_t lut_off;          // where the warps keep their LUT rows at 4 to 7 bits (aligned to kApLutStride)
     uint32_t smem_bytes;
     uint32_t direct;           // 1: fold into y; 0: store into the accumulator and take the tile's ticket
     uint32_t wait_ns;          // limit of one mbarrier wait (DECDEC_PIPE_WAIT_NS)
@@ -51,10 +51,12 @@ struct ApPipeGeom {
 constexpr int kApPipeHdr = 256;   // [abort, flag][full barriers 8][empty barriers 8]
 
 // One plane-word position (32 channels) of one row through the lookup decoder: W[jj][i] = weights of channels 2i (low half) and
-// 2i + 1 of group jj, beside the activations as they lie in memory.  `lut` is the window address of the row's LUT, aligned to
-// kApLutStride.  Up to 7 bits the byte offset of an entry, 2 * code, fits a byte: even and odd nibble positions are moved
-// into the bytes of two words (E and O), and one byte permute puts such a byte under the upper bytes of `lut`.
-template <int BITS> constexpr uint32_t kApLutStride = BITS <= 7 ? 256u : 512u;
+// 2i + 1 of group jj, beside the activations as they lie in memory.  `lut` is the window address of the row's LUT.  Even and odd
+// nibble positions are moved into the bytes of two words (E and O).  Up to 7 bits such a byte holds the byte offset of an entry,
+// 2 * code, and one byte permute puts it under the upper bytes of `lut`, which is aligned to kApLutStride.  At 8 bits it holds
+// the code; a permute takes it out and `lut`, where the copy landed it, is added: 512 bytes per row are too much to move again in
+// every warp (768 x 4096 7.5 us, 5.0 without).
+constexpr uint32_t kApLutStride = 256;
 
 template <int BITS>
 __device__ __forceinline__ void ap_lookup_word(const uint32_t* q, uint32_t lut, uint32_t (&W)[4][4]) {
@@ -78,7 +80,7 @@ __device__ __forceinline__ void ap_lookup_word(const uint32_t* q, uint32_t lut, 
         const int b = t >> 1;
         uint32_t addr;
         if constexpr (BITS <= 7) addr = __byte_perm(src, lut, 0x7650u | (uint32_t)b);
-        else addr = (b ? (src >> (8 * b - 1)) & 0x1feu : (src << 1) & 0x1feu) | lut;
+        else addr = lut + 2u * __byte_perm(src, 0u, 0x4440u | (uint32_t)b);
         uint16_t v;
         asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
         return v;
@@ -181,8 +183,8 @@ __device__ void ap_pipe_role(const ApParams& p, const FinParams& f, const ApPipe
         const uint32_t full = nseg / 32u;
         const uint32_t g = lane >> 2;
         const bool diag = (lane & 3u) == (g >> 1), odd = (g & 1u) != 0u;
-        const uint32_t lutA = smem_u32(sm) + geo.lut_off + warp * 2u * kApLutStride<BITS>;
-        uint32_t* lut_own = reinterpret_cast<uint32_t*>(sm + geo.lut_off + (size_t)warp * 2u * kApLutStride<BITS>);
+        const uint32_t lut_mine = smem_u32(sm) + geo.lut_off + warp * 2u * kApLutStride;       // 4 to 7 bits
+        uint32_t* lut_own = reinterpret_cast<uint32_t*>(sm + geo.lut_off + (size_t)warp * 2u * kApLutStride);
 
         for (uint32_t i = 0; i < nst; ++i) {
             const uint32_t s = i % S;
@@ -199,15 +201,17 @@ __device__ void ap_pipe_role(const ApParams& p, const FinParams& f, const ApPipe
                     const uint4 b = *reinterpret_cast<const uint4*>(st + lut_off + rowB * kLutRow);
                     tA.fill_pairs(&a.x);
                     tB.fill_pairs(&b.x);
-                } else {
+                } else if constexpr (BITS <= 7) {
                     // the pair's LUT rows to the warp's own, aligned place
                     __syncwarp();
                     const uint32_t* lw = reinterpret_cast<const uint32_t*>(st + lut_off + rowA * kLutRow);
                     constexpr uint32_t half = kLutRow / 4u;
                     const uint32_t n_lw = rowB > rowA ? 2u * half : half;
-                    for (uint32_t at = lane; at < n_lw; at += 32u) lut_own[at < half ? at : at - half + kApLutStride<BITS> / 4u] = lw[at];
+                    for (uint32_t at = lane; at < n_lw; at += 32u) lut_own[at < half ? at : at - half + kApLutStride / 4u] = lw[at];
                     __syncwarp();
                 }
+                const uint32_t lutA = BITS <= 7 ? lut_mine : smem_u32(st) + lut_off + rowA * kLutRow;
+                const uint32_t lutB = BITS <= 7 ? lut_mine + kApLutStride : lutA + (rowB - rowA) * kLutRow;
                 // RAGGED: the last step of a segment that is not a whole number of 32 words.  Lanes without one add zero
                 // weights, not table entries that zero activations might turn into NaN.
                 auto step = [&](uint32_t u, auto RAGGED) {
@@ -230,7 +234,7 @@ __device__ void ap_pipe_role(const ApParams& p, const FinParams& f, const ApPipe
                     if constexpr (LOOKUP) {
                         uint32_t WA[4][4], WB[4][4];
                         ap_lookup_word<BITS>(qA, lutA, WA);
-                        ap_lookup_word<BITS>(qB, lutA + kApLutStride<BITS>, WB);
+                        ap_lookup_word<BITS>(qB, lutB, WB);
                         if constexpr (RAGGED.value) {
 #pragma unroll
                             for (int jj = 0; jj < 4; ++jj)

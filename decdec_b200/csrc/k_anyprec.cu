@@ -46,7 +46,7 @@ template <int DT, int BITS>
 __global__ void __launch_bounds__(kApPipeThreads, 1)
 k_anyprec_pipe(const __grid_constant__ ApParams g, const __grid_constant__ DecParams d, const __grid_constant__ FinParams f,
                const __grid_constant__ ApPipeGeom geo) {
-    extern __shared__ __align__(512) unsigned char sm[];     // the warps' LUT rows are aligned to kApLutStride
+    extern __shared__ __align__(256) unsigned char sm[];     // the warps' LUT rows are aligned to kApLutStride
     if (blockIdx.x < d.n_cta) dec_role<DT>(d, f, blockIdx.x, sm);
     else ap_pipe_role<DT, BITS>(g, f, geo, blockIdx.x - d.n_cta, sm);
 }
@@ -65,8 +65,8 @@ bool anyprec_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, ApPipeGeom* ge
     const uint32_t gran = gemv_only ? 16u : 32u;
     rows = ((rows + gran - 1) / gran) * gran;
     geo->rows_per_cta = rows;
-    const uint32_t lut_stride = bits <= 7 ? kApLutStride<7> : kApLutStride<8>;
-    const uint32_t lut_bytes = bits > 3 ? 16u * 2u * lut_stride + lut_stride : 0u;       // 16 warps, and room for the alignment
+    const bool own_luts = bits > 3 && bits < 8;
+    const uint32_t lut_bytes = own_luts ? 16u * 2u * kApLutStride + kApLutStride : 0u;   // 16 warps, and room for the alignment
     // Cut of a stage over the 16 warps: rows in pairs, a row's 1024-channel blocks in `segs` segments.  A stage costs its
     // warps the blocks of a segment plus about 0.8 of a block for the wait, the tables and the sums; long segments spread
     // that best, short ones fill the warps when the CTA has few rows (and leave room for two stages of wide rows).
@@ -98,8 +98,8 @@ bool anyprec_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, ApPipeGeom* ge
         geo->stage_bytes = stage;
         geo->stages = nst < smax ? nst : smax;
         const uint32_t end = kApPipeHdr + geo->x_bytes + part + geo->stages * stage;
-        geo->lut_off = (end + lut_stride - 1u) & ~(lut_stride - 1u);
-        geo->smem_bytes = bits > 3 ? geo->lut_off + 16u * 2u * lut_stride : end;
+        geo->lut_off = (end + kApLutStride - 1u) & ~(kApLutStride - 1u);
+        geo->smem_bytes = own_luts ? geo->lut_off + 16u * 2u * kApLutStride : end;
     }
     if (best == 0xffffffffu) return false;
     geo->direct = 0;        // set by the caller
