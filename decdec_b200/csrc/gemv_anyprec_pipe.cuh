@@ -11,13 +11,15 @@
 //    D[g][g] and D[g + 8][g] hold the sums of the quad's lanes for the two rows; the other entries mix lanes and are not used.
 //    One instruction consumes eight weights per lane, and nothing is summed in 16 bits;
 //  * the eight diagonal sums of a row are stored, not shuffled together: the fold at the end adds a row's slots, in a fixed order;
-//  * the loop over a row's 1024-channel blocks is not unrolled (unrolled twice: the same times), and the last, shorter block has
-//    a body of its own, so that the masks it needs are not paid for by the others.
-// Measured, fp16, us per launch in a graph on 28672 x 4096, against the same stages with packed 16-bit sums (3 bits) or two
-// address operations and one mixed-precision multiply-add per weight (4 to 8 bits): 3 bits 24.2 -> 23.6, 4 bits 39.9 -> 30.0,
-// 5 bits 54.1 -> 33.8, 6 bits 55.5 -> 34.7, 8 bits 61.2 -> 57.9 (1.9, 2.0, 2.2, 2.6 and 2.3 TB/s of algorithmic bytes).
+//  * the loop over a row's 1024-channel blocks is unrolled twice at 3 bits (28672 x 4096 23.1 -> 22.7 us; at 4 to 8 bits small layers
+//    lose by it: 512 x 1792 at 8 bits 3.5 -> 3.8), and the last, shorter block has a body of its own, so that the masks it needs
+//    are not paid for by the others.
+// Measured, fp16, us per launch in a graph, against the same stages with packed 16-bit sums (3 bits) or two address operations and
+// one mixed-precision multiply-add per weight (4 to 8 bits): on 28672 x 4096 3 bits 22.7 -> 22.7, 4 bits 37.6 -> 29.3, 8 bits
+// 57.9 -> 53.3 (2.0, 2.0 and 2.2 TB/s of algorithmic bytes); on 4096 x 14336 16.1 -> 12.6, 25.5 -> 19.3, 37.0 -> 31.2; on
+// 768 x 4096 3.6 -> 3.1, 4.9 -> 3.7, 6.5 -> 4.8.
 // Two decoders.  3 bits: the row's table lives in registers and is looked up by byte permutes (lut_bytes.cuh), activations staged
-// in the pair order the lookups produce.  4 to 8 bits: the plane words are regrouped into 4-bit fields, each code indexes the
+// in the order in which the products take them.  4 to 8 bits: the plane words are regrouped into 4-bit fields, each code indexes the
 // row's LUT in shared memory (a row of up to 64 entries spans at most 32 banks and equal entries broadcast, so a
 // lookup is one wavefront).
 // A CTA owns its rows completely (all of K) and folds them into y itself: GEMV-only launches use no global accumulator, ticket
@@ -40,7 +42,7 @@ struct ApPipeGeom {
     uint32_t stages;           // pipeline depth
     uint32_t stage_bytes;
     uint32_t x_bytes;          // staged activations (rounded to 128)
-    uint32_t rows_per_cta;     // multiple of R
+    uint32_t rows_per_cta;     // even; a multiple of 32 beside a compensation role
     uint32_t part_bytes;       // partial sums of the CTA: fp32 [row][segment][8]
     uint32_t lut_off;          // where the warps keep their LUT rows at 4 to 7 bits (aligned to kApLutStride)
     uint32_t smem_bytes;
@@ -168,11 +170,37 @@ __device__ void ap_pipe_role(const ApParams& p, const FinParams& f, const ApPipe
         // ------------------------------ consumers ----------------------------------------------
         pdl_wait();     // weights are already streaming (producer warp); activations come from earlier kernels
         const T* x = reinterpret_cast<const T*>(p.x);
-        // the byte-permute decoder delivers channel pairs (7 - i, 3 - i): its activations are staged in that order
-        for (uint32_t k = tid; k < p.K; k += NW * 32) sx[LOOKUP ? k : ((k & ~7u) | ap_perm(k & 7u))] = x[k];
+        const uint32_t tailE = nwords & 31u;              // words of the row's last, shorter block
+        if constexpr (LOOKUP) {
+            for (uint32_t k = tid; k < p.K; k += NW * 32) sx[k] = x[k];
+        } else {
+            // the byte-permute decoder delivers, for every ph, the channel pairs (7 - ph, 3 - ph) of the four groups of a word:
+            // their activations are staged side by side, groups 3 to 0, where a group's eight channels lie in memory.  One load of
+            // the main loop then holds both operand registers of two instructions, in the right order.
+            const bool xvec = (reinterpret_cast<uintptr_t>(x) & 15u) == 0u;
+            for (uint32_t w = tid; w < nwords; w += NW * 32) {
+                const uint32_t E = (w >> 5) == (nwords >> 5) ? tailE : 32u;
+                const uint32_t at = (w & ~31u) * 32u + 8u * (w & 31u);
+                union { uint4 v; unsigned short e[8]; } q[4];
+#pragma unroll
+                for (int jj = 0; jj < 4; ++jj) {
+                    const unsigned short* src = reinterpret_cast<const unsigned short*>(x) + at + 8u * E * jj;
+                    if (xvec) q[jj].v = *reinterpret_cast<const uint4*>(src);
+                    else
+#pragma unroll
+                        for (int r = 0; r < 8; ++r) q[jj].e[r] = src[r];
+                }
+#pragma unroll
+                for (int ph = 0; ph < 4; ++ph) {
+                    uint32_t o[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) o[i] = (uint32_t)q[3 - i].e[7 - ph] | ((uint32_t)q[3 - i].e[3 - ph] << 16);
+                    *reinterpret_cast<uint4*>(sx + at + 8u * E * ph) = make_uint4(o[0], o[1], o[2], o[3]);
+                }
+            }
+        }
         asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
 
-        const uint32_t tailE = nwords & 31u;              // words of the row's last, shorter block
         const uint32_t pair = warp / geo.segs, seg = warp % geo.segs;
         const uint32_t rowA = 2u * pair, rowB = min(rowA + 1u, R - 1u);   // a stage of one row: its sums are formed twice, used once
         const bool has_item = rowA < R;
@@ -262,12 +290,12 @@ __device__ void ap_pipe_role(const ApParams& p, const FinParams& f, const ApPipe
                             tA.lookup(VA[ph] >> 16, a1, a0);
                             tB.lookup(VB[ph], b3, b2);
                             tB.lookup(VB[ph] >> 16, b1, b0);
-                            mma_16816<DT>(acc[0], a3, b3, a2, b2, (&X[3].x)[ph], (&X[2].x)[ph]);
-                            mma_16816<DT>(acc[1], a1, b1, a0, b0, (&X[1].x)[ph], (&X[0].x)[ph]);
+                            mma_16816<DT>(acc[0], a3, b3, a2, b2, X[ph].x, X[ph].y);
+                            mma_16816<DT>(acc[1], a1, b1, a0, b0, X[ph].z, X[ph].w);
                         }
                     }
                 };
-#pragma unroll 1
+#pragma unroll (LOOKUP ? 1 : 2)
                 for (uint32_t u = 0; u < full; ++u) step(u, IsRagged<false>{});
                 if (full * 32u < nseg) step(full, IsRagged<true>{});
             }

@@ -53,8 +53,8 @@ k_anyprec_pipe(const __grid_constant__ ApParams g, const __grid_constant__ DecPa
 
 // Stage geometry of the pipelined kernel (3 to 8 bits); false if the shape is not eligible.  A CTA's rows are a whole
 // number of 32-output finalizer tiles when a compensation role may share the launch; a GEMV-only launch (no config)
-// has no finalizer and cuts the rows in multiples of 16, which fills the SMs more evenly (6144 rows: 128 CTAs of 48
-// instead of 96 of 64).
+// has no finalizer and cuts the rows in pairs, which fills the SMs evenly (us at 3 bits, rows in multiples of 16 -> in pairs:
+// 768 x 4096 3.94 -> 3.31, 1000 x 2176 4.00 -> 3.28, 4096 x 14336 14.65 -> 13.52, 28672 x 4096 23.53 -> 23.36).
 bool anyprec_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, ApPipeGeom* geo, uint32_t sm_budget, bool gemv_only) {
     if (bits < 3 || bits > 8 || K % 128u || K > 32768u || N == 0) return false;
     const uint32_t rowbytes = K / 8;
@@ -62,7 +62,7 @@ bool anyprec_pipe_geometry(uint32_t N, uint32_t K, uint32_t bits, ApPipeGeom* ge
     geo->x_bytes = (K * 2 + 127u) & ~127u;
     if (sm_budget == 0) sm_budget = 1;
     uint32_t rows = (N + sm_budget - 1) / sm_budget;
-    const uint32_t gran = gemv_only ? 16u : 32u;
+    const uint32_t gran = gemv_only ? 2u : 32u;
     rows = ((rows + gran - 1) / gran) * gran;
     geo->rows_per_cta = rows;
     const bool own_luts = bits > 3 && bits < 8;
