@@ -57,7 +57,7 @@ __device__ __forceinline__ float bucket_floor(float a_f, float b_f, int L) {
 // The smallest floor up to each bucket, into shared memory: bucket(e) = the first L with floor[L] <= |x_e| is then the first L with
 // smallest[L] <= |x_e|, and that sequence never rises, whatever the thresholds are, so it can be searched.  Depends on the
 // launch's arguments alone: done before the wait for the previous kernel, once for all chunks of a CTA.
-// Five dependent loads replace 32 comparisons and mask operations per channel, which were most of the selection's 2.4 us; with the
+// Six dependent loads replace 32 comparisons and mask operations per channel, which were most of the selection's 2.4 us; with the
 // floors out of the chain as well, the eight fused launches of two 8B blocks went from 224 to 217 us at 32 channels per 1024
 // and from 96.8 to 91.7 us at (0, 0, 5, 3).
 template <int DT>

@@ -1,8 +1,8 @@
-"""CPU check of the index arithmetic of the any-precision lookup decoder (`csrc/gemv_anyprec_pipe.cuh`:
-`ap_fields`, `ap_lookup_word`), restated in Python with the same shifts and masks, against the oracle's packer of the
+"""CPU check of the index arithmetic of the any-precision decoders (`csrc/lut_bytes.cuh`: `ap_fields`; `csrc/gemv_anyprec.cuh`:
+`ap_dequant_kernel`; `csrc/gemv_anyprec_pipe.cuh`: `ap_lookup_word`), restated in Python with the same shifts and masks, against the oracle's packer of the
 reference layout (`decdec_extension/anyprec.cu:261-331`: bit 31-8j-r of word t of a block holds channel
 block_start + 8*E*j + 8*t + r, plane 0 is the most significant code bit).  The kernel itself is compared with the oracle
-on the GPU (`tests/test_gpu_parity.py::test_anyprec_gemv`); this test pins the regrouping where no GPU is present."""
+on the GPU (`tests/test_gpu_parity.py::test_anyprec_gemv`, `tests/test_gpu_lut_paths.py`); this test pins the regrouping where no GPU is present."""
 import numpy as np
 import pytest
 
@@ -35,7 +35,7 @@ def fields(planes):
 
 
 def word_codes(q, bits):
-    """ap_lookup_word: {(j, r): code} for the 32 channels of one plane-word position, from the byte offsets the kernel forms."""
+    """ap_dequant_kernel: {(j, r): code} for the 32 channels of one plane-word position, from the nibbles of both field sets."""
     bh = min(bits, 4)
     bl = bits - bh
     vh = fields(q[:bh])
@@ -45,21 +45,17 @@ def word_codes(q, bits):
         for t in range(8):
             pos = 31 - (4 * t + ph)
             j, r = pos >> 3, pos & 7
-            if bl == 0:
-                off = ((vh[ph] >> (4 * t - 1)) & 0x1E) if t else ((vh[ph] << 1) & 0x1E)
-            else:
-                mh, ml = 0xF << (bl + 1), ((1 << bl) - 1) << 1
-                sh = 4 * t - bl - 1
-                off = ((vh[ph] >> sh) if sh >= 0 else (vh[ph] << -sh)) & mh
-                off |= ((vl[ph] >> (4 * t - 1)) if t else (vl[ph] << 1)) & ml
-            assert off % 2 == 0 and off < (2 << bits)
-            codes[(j, r)] = off >> 1
+            code = (vh[ph] >> (4 * t)) & 0xF
+            if bl:
+                code = (code << bl) | ((vl[ph] >> (4 * t)) & ((1 << bl) - 1))
+            assert code < (1 << bits)
+            codes[(j, r)] = code
     return codes
 
 
 @pytest.mark.parametrize("bits", [3, 4, 5, 6, 7, 8])
 @pytest.mark.parametrize("K", [128, 1024, 1536])
-def test_lookup_offsets_recover_the_packed_codes(bits, K):
+def test_dequantizer_fields_recover_the_packed_codes(bits, K):
     rng = np.random.default_rng(bits * 100 + K)
     N = 2
     want = rng.integers(0, 2 ** bits, size=(N, K)).astype(np.int32)
