@@ -15,8 +15,8 @@
 //    lose by it: 512 x 1792 at 8 bits 3.5 -> 3.8), and the last, shorter block has a body of its own, so that the masks it needs
 //    are not paid for by the others.
 // Measured, fp16, us per launch in a graph, against the same stages with packed 16-bit sums (3 bits) or two address operations and
-// one mixed-precision multiply-add per weight (4 to 8 bits): on 28672 x 4096 3 bits 22.7 -> 22.7, 4 bits 37.6 -> 29.3, 8 bits
-// 57.9 -> 53.3 (2.0, 2.0 and 2.2 TB/s of algorithmic bytes); on 4096 x 14336 16.1 -> 12.6, 25.5 -> 19.3, 37.0 -> 31.2; on
+// one mixed-precision multiply-add per weight (4 to 8 bits): on 28672 x 4096 3 bits 22.7 -> 22.7, 4 bits 37.6 -> 29.3, 5 bits
+// 51.1 -> 33.1, 6 bits 52.4 -> 34.4, 8 bits 57.9 -> 53.4 (2.0, 2.0, 2.2, 2.6 and 2.5 TB/s of algorithmic bytes); on 4096 x 14336 16.1 -> 12.6, 25.5 -> 19.3, 37.0 -> 31.2; on
 // 768 x 4096 3.6 -> 3.1, 4.9 -> 3.7, 6.5 -> 4.8.
 // Two decoders.  3 bits: the row's table lives in registers and is looked up by byte permutes (lut_bytes.cuh), activations staged
 // in the order in which the products take them.  4 to 8 bits: the plane words are regrouped into 4-bit fields, each code indexes the

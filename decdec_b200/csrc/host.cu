@@ -389,8 +389,11 @@ int run_anyprec(Config* c, const void* x, void* y, const int32_t* qw, uint32_t p
     uint32_t budget = gemv_sm_budget(c, true);
     if (c) {
         // many compensation thread blocks (the launch is bound by the host link): the GEMV runs in the SMs they leave
-        // free and takes over the rest as they retire, which it does more evenly in thread blocks half the size (eight fused
-        // 4-bit launches of two 8B blocks at k_chunk 8: 220 / 214 / 228 us for one, two and three)
+        // free and takes over the rest as they retire, which it does more evenly in thread blocks half the size.  us for one, two
+        // and three times as many, 28672 x 4096: 3 bits, k_chunk 8, n_tb 48 40.2 / 32.7 / 37.2 and n_tb 96 40.9 / 41.7 / 39.6, k_chunk 32,
+        // n_tb 48 49.7 / 46.4 / 49.6 and n_tb 96 68.1 / 58.1 / 60.0; 4 bits 47.1 / 41.3 / 48.1, 47.8 / 49.5 / 48.3, 60.3 / 56.8 / 50.7
+        // and 75.9 / 63.5 / 66.2.  4096 x 4096 and 4096 x 14336 take the same times with all three, 6144 x 4096 11.0 / 13.5 / 13.3 at
+        // 3 bits, k_chunk 8, n_tb 48 but 17.8 / 16.3 / 16.3 at n_tb 96.
         DecParams dg;
         memset(&dg, 0, sizeof(dg));
         dec_geometry(c, true, 1u << 20, &dg);
