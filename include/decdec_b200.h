@@ -18,7 +18,8 @@
  *     device allocates (its own and sixteen spare ones, 2 MB each) and therefore must not happen during stream capture.
  *     A stream first seen while it is capturing takes a spare; when the spares are used up it shares the
  *     device's first workspace, and that graph must then not run concurrently with work on the owning stream.
- *     Calls that share a stream are ordered; calls on different streams use different workspaces.
+ *     Calls that share a stream are ordered; calls on different streams use different workspaces.  Graphs captured on
+ *     one stream share its workspace and must not be replayed at the same time.
  */
 #ifndef DECDEC_B200_H
 #define DECDEC_B200_H
