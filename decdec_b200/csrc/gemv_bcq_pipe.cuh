@@ -228,15 +228,16 @@ __device__ void bcq_pipe_role(const BcqParams& p, const FinParams& f, const Pipe
             // ragged layers are ordered like plain launches: their weights may come from the kernel before
             if (RAGGED) pdl_wait();
             for (uint32_t i = 0; i < n_issue; ++i) {
-                const uint32_t s = ring_place(i, S, geo.inv_stages);
-                if (i >= S) {
+                // the consumers' numbers (stage_ring.h), by division: see there
+                const uint32_t s = i % S, use = i / S;
+                if (use > 0) {
                     // A slot frees only after the consumers have passed their own wait for the previous kernel, which
                     // may itself be waiting for another GPU: the bounded wait must not run during that time.  Every
                     // slot is full at this point, so waiting for the dependency here delays no copy.
-                    if (i == S) pdl_wait();
-                    if (!mbar_wait(bar_empty + 8 * s, ring_parity(i - S, geo.inv_stages), s_abort, geo.wait_ns)) break;
+                    if (use == 1 && s == 0) pdl_wait();
+                    if (!mbar_wait(bar_empty + 8 * s, (use - 1) & 1u, s_abort, geo.wait_ns)) break;
                 }
-                const uint32_t full = bar_full + 8 * ring_place(i, geo.fulls, geo.inv_fulls);
+                const uint32_t full = bar_full + 8 * (i % geo.fulls);
                 mbar_expect_tx(full, tx);
                 const uint32_t n0 = (st0 + i) * kPipeStageN;
                 const uint32_t dst = smem_u32(stage_ptr(s));

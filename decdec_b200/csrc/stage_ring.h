@@ -13,9 +13,10 @@
 // One `full` barrier per slot is not enough for other S.  With 2 slots and 3 groups, group 2 starts at stage 2 and finds slot 0's
 // barrier in phase 0, which its parity cannot tell from phase 1 completed: it reads a slot that is being written.  With 4 slots it
 // takes a first copy that lands after a later one's group is done.
-// Measured (us, fp16, sixteen launches of four 8B blocks, 3 bits, S = 5, and 28672 x 4096 at 4 bits, S = 3; one barrier per slot: 143.6
-// and 20.4): this 141.8 and 21.2; two barriers per slot for every S and as many groups as slots 142.2 and 21.7; consumers that
-// wait for `free` as well 149.5.
+// Measured (us, fp16, 28672 x 4096 at 2, 3 and 4 bits: 8, 5 and 3 slots; one barrier per slot 12.1, 15.2 and 20.4): this 11.8, 14.8 and
+// 20.5.  The consumers, who are short of registers, find places by multiplication, the producer by division: with divisions on
+// both sides 12.4, 15.4 and 21.6, with multiplications 12.0, 14.9 and 21.4.  Two barriers per slot for every S and as many groups as
+// slots 12.3, 14.8 and 21.9; consumers that wait for `free` as well 4 % more over the launches of an 8B block.
 #pragma once
 #include <stdint.h>
 
